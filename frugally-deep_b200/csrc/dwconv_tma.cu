@@ -475,6 +475,12 @@ void launch_pool_tiles(const float* in, float* out, int64_t B, int H, int W, int
     else launch_pool_variant<3, 1, 7>(is_max, grid, threads, smem, map, p, s);
 }
 
+const int* dwconv_tiles_status_address() {
+    int* p = nullptr;
+    FDK_CUDA(cudaGetSymbolAddress((void**)&p, g_dw_status));
+    return p;
+}
+
 int dwconv_tiles_take_status(cudaStream_t s) {
     int v = 0;
     if (cudaMemcpyFromSymbolAsync(&v, g_dw_status, sizeof(int), 0, cudaMemcpyDeviceToHost, s) != cudaSuccess) { cudaGetLastError(); return 0; }

@@ -1,11 +1,13 @@
 // Executor: device contexts, weight upload, plan execution, predict_multi sharding.
 #include "engine.hpp"
+#include "copy_pool.hpp"
 #include "kernels.cuh"
 #include "plan_attrs.hpp"
 
 #include <algorithm>
 #include <atomic>
 #include <cmath>
+#include <cstdlib>
 #include <cstring>
 #include <thread>
 
@@ -60,10 +62,13 @@ Engine::Engine(LoadedModel&& lm, const std::vector<int>& devices, const EngineOp
         FDK_CUDA(cudaEventCreateWithFlags(&c->fork_event, cudaEventDisableTiming));
         FDK_CUDA(cudaEventCreateWithFlags(&c->join_event, cudaEventDisableTiming));
         FDK_CUDA(cudaEventCreateWithFlags(&c->busy, cudaEventDisableTiming));
-        FDK_CUDA(cudaMalloc(&c->d_err, sizeof(int)));
-        FDK_CUDA(cudaMemset(c->d_err, 0, sizeof(int)));
-        FDK_CUDA(cudaMallocHost(&c->h_err, sizeof(int)));
-        *c->h_err = 0;
+        FDK_CUDA(cudaMalloc(&c->d_err, 2 * sizeof(int)));
+        FDK_CUDA(cudaMemset(c->d_err, 0, 2 * sizeof(int)));
+        FDK_CUDA(cudaMallocHost(&c->h_err, 8 * sizeof(int)));
+        std::memset(c->h_err, 0, 8 * sizeof(int));
+        c->status[0] = gemm_tc_status_address();
+        c->status[1] = gemm_rows_status_address();
+        c->status[2] = dwconv_tiles_status_address();
         upload_weights(*c);
         ctx_.push_back(std::move(c));
     }
@@ -75,6 +80,7 @@ Engine::~Engine() {
         cudaStreamSynchronize(c->stream);
         if (c->busy_valid) cudaEventSynchronize(c->busy);
         if (c->busy) cudaEventDestroy(c->busy);
+        for (auto& r : c->calls) if (r.exec) cudaGraphExecDestroy(r.exec);
         cudaFree(c->w.base);
         cudaFree(c->arena);
         cudaFree(c->in_stage);
@@ -270,6 +276,8 @@ struct Exec {
     std::vector<int> norm_of_op;      // per operation: the normalisation its products apply to their input first, or -1
     std::vector<char> norm_folded;    // per operation: 1 = this normalisation runs inside its consumer and is not launched
     const std::vector<char>* wanted = nullptr;   // per plan output: 0 = the caller does not want it (null: all wanted)
+    std::vector<float*> bound;                   // per buffer: the caller's output memory it lives in (empty: all in the arena)
+    int* err = nullptr;                          // flag of the device-side input checks
     // profiling (off unless `prof` is set): events around operations and contraction launches
     struct Rec { std::string kind, name, path; cudaEvent_t a, b; double flops; int64_t M; int N, K; };
     std::vector<Rec>* prof = nullptr;
@@ -285,6 +293,7 @@ struct Exec {
     float* tptr(int t) const {
         const BufferInfo& b = p.buffers[(size_t)p.tensors[(size_t)t].buf];
         if (b.ext_input >= 0) return const_cast<float*>(d_in[b.ext_input]);
+        if (!bound.empty() && bound[(size_t)p.tensors[(size_t)t].buf]) return bound[(size_t)p.tensors[(size_t)t].buf];
         return c.arena + b.offset * B;
     }
     float* bptr(int buf) const { return c.arena + p.buffers[(size_t)buf].offset * B; }
@@ -588,7 +597,7 @@ struct Exec {
                 }
                 case OP_EMBED:
                     launch_embedding(tptr(o.in[0]), wptr(o.layer->w_main), tptr(o.out[0]), B * shape(o.in[0]).d[4], o.layer->units,
-                                     o.layer->input_dim, c.d_err, s);
+                                     o.layer->input_dim, err, s);
                     c.launches++;
                     break;
                 case OP_LSTM:
@@ -704,7 +713,7 @@ struct Exec {
                     c.launches++;
                     break;
                 case OP_LOOKUP:
-                    launch_lookup((int)o.a[0], tptr(o.in[0]), tptr(o.out[0]), wptr(o.layer->w_main), B, o.a[2], (int)o.a[1], o.a[3] != 0, c.d_err, s);
+                    launch_lookup((int)o.a[0], tptr(o.in[0]), tptr(o.out[0]), wptr(o.layer->w_main), B, o.a[2], (int)o.a[1], o.a[3] != 0, err, s);
                     c.launches++;
                     break;
                 case OP_CONVLSTM_CELL:
@@ -1039,14 +1048,34 @@ struct Exec {
 };
 }  // namespace
 
+// The caller's memory takes the place of an output's buffer in the arena when it can: the buffer holds exactly that output
+// (not a part, not an input handed through), the memory is aligned as the kernels' vector and TMA stores want it, and it is
+// none of the call's inputs.
+static bool bound_output(const Plan& p, size_t o, const float* d_out, int64_t batch, const float* const* d_in) {
+    for (size_t i = 0; i < p.inputs.size(); ++i)
+        if (d_out && d_in[i] < d_out + batch * p.tensors[(size_t)p.outputs[o]].shape.volume() && d_out < d_in[i] + batch * p.in_shapes[i].volume()) return false;
+    const TensorInfo& t = p.tensors[(size_t)p.outputs[o]];
+    const BufferInfo& b = p.buffers[(size_t)t.buf];
+    if (!d_out || b.ext_input >= 0 || b.elems != t.shape.volume() || (reinterpret_cast<uintptr_t>(d_out) & 255) != 0) return false;
+    for (size_t k = 0; k < o; ++k)
+        if (p.tensors[(size_t)p.outputs[k]].buf == t.buf) return false;   // the first of several views
+    return true;
+}
+
 void Engine::execute(DeviceCtx& c, const Plan& p, int64_t B, const float* const* d_in, cudaStream_t s, std::string* profile, const KvCache* kv,
-                     const std::vector<char>* wanted) {
+                     const std::vector<char>* wanted, float* const* d_out, int* err) {
     ensure_arena(c, std::max<int64_t>(p.arena_elems, 64) * B);
     Exec ex{*this, c, p, B, d_in, s, opt_.use_tc};
     ex.use_skinny = opt_.skinny;
     ex.fuse_cells = opt_.fuse_cells;
     ex.kv = kv;
     ex.wanted = wanted;
+    ex.err = err ? err : c.d_err;
+    if (d_out) {
+        ex.bound.assign(p.buffers.size(), nullptr);
+        for (size_t o = 0; o < p.outputs.size(); ++o)
+            if (bound_output(p, o, d_out[o], B, d_in)) ex.bound[(size_t)p.tensors[(size_t)p.outputs[o]].buf] = d_out[o];
+    }
     std::vector<Exec::Rec> recs;
     if (profile) ex.prof = &recs;
     ex.run();
@@ -1111,15 +1140,97 @@ void Engine::predict_batch_device(int dev_index, int64_t batch, const float* con
     if (live) order_after_last_use(c, s);
     std::vector<char> wanted(p->outputs.size(), 1);
     for (size_t o = 0; o < p->outputs.size(); ++o) wanted[o] = d_out[o] != nullptr ? 1 : 0;
-    execute(c, *p, batch, d_in, s, profile, kv, &wanted);
-    for (size_t o = 0; o < p->outputs.size(); ++o) {
-        const TensorInfo& t = p->tensors[(size_t)p->outputs[o]];
-        const BufferInfo& b = p->buffers[(size_t)t.buf];
-        const float* src = b.ext_input >= 0 ? d_in[b.ext_input] : c.arena + b.offset * batch;
-        if (!d_out[o]) continue;  // output not wanted
-        FDK_CUDA(cudaMemcpyAsync(d_out[o], src, sizeof(float) * (size_t)(batch * t.shape.volume()), cudaMemcpyDeviceToDevice, s));
+    auto queue = [&](cudaStream_t on) {
+        execute(c, *p, batch, d_in, on, profile, kv, &wanted, d_out);
+        for (size_t o = 0; o < p->outputs.size(); ++o) {
+            if (!d_out[o] || bound_output(*p, o, d_out[o], batch, d_in)) continue;  // output not wanted, or written by its kernel
+            const TensorInfo& t = p->tensors[(size_t)p->outputs[o]];
+            const BufferInfo& b = p->buffers[(size_t)t.buf];
+            const float* src = b.ext_input >= 0 ? d_in[b.ext_input] : c.arena + b.offset * batch;
+            for (size_t k = 0; k < o; ++k)   // another view of an output that lives in the caller's memory
+                if (p->tensors[(size_t)p->outputs[k]].buf == t.buf && bound_output(*p, k, d_out[k], batch, d_in)) src = d_out[k];
+            FDK_CUDA(cudaMemcpyAsync(d_out[o], src, sizeof(float) * (size_t)(batch * t.shape.volume()), cudaMemcpyDeviceToDevice, on));
+        }
+    };
+    if (!live || profile || kv) {
+        queue(s);
+    } else {
+        std::vector<const void*> where(d_in, d_in + p->inputs.size());
+        where.insert(where.end(), d_out, d_out + p->outputs.size());
+        replay(c, *p, batch, std::move(where), 0.f, 0.f, s, queue);
     }
     if (live) mark_use(c, s);
+}
+
+// A call repeated with the same plan, batch and addresses costs one graph launch instead of the launches of the plan (60 to
+// 800 of them, 3 to 6 us of host time each with their tensor maps, and gaps between short kernels).  The first call of a kind
+// runs directly (every buffer reaches its size), the second one is recorded.  At most 32 calls are kept per device; the
+// addresses of the arena and the workspace belong to the key because other calls may make them move.
+template <typename F>
+void Engine::replay(DeviceCtx& c, const Plan& p, int64_t batch, std::vector<const void*> where, float low, float high, cudaStream_t s, F&& queue) {
+    static const bool enabled = [] { const char* v = getenv("FDK_PREDICT_GRAPH"); return !(v && *v == '0'); }();
+    if (!enabled) {
+        queue(s);
+        return;
+    }
+    where.push_back(c.arena);
+    where.push_back(c.workspace);
+    RecordedCall* r = nullptr;
+    for (auto& k : c.calls)
+        if (k.plan == &p && k.batch == batch && k.low == low && k.high == high && k.where == where) r = &k;
+    if (!r) {
+        queue(s);
+        if (where[where.size() - 2] != c.arena || where.back() != c.workspace) return;   // they moved: not this kind's steady state yet
+        if (c.calls.size() >= 32) {
+            auto oldest = std::min_element(c.calls.begin(), c.calls.end(), [](const RecordedCall& x, const RecordedCall& y) { return x.last_use < y.last_use; });
+            if (oldest->exec) cudaGraphExecDestroy(oldest->exec);
+            c.calls.erase(oldest);
+        }
+        RecordedCall k;
+        k.plan = &p; k.batch = batch; k.low = low; k.high = high;
+        k.where = std::move(where);
+        k.last_use = ++c.call_clock;
+        c.calls.push_back(std::move(k));
+        return;
+    }
+    r->last_use = ++c.call_clock;
+    if (!r->exec && !r->unusable) {
+        const int64_t before = c.launches;
+        cudaGraph_t graph = nullptr;
+        FDK_CUDA(cudaStreamBeginCapture(c.stream, cudaStreamCaptureModeRelaxed));
+        bool ok = true;
+        try {
+            queue(c.stream);
+        } catch (const std::exception&) {
+            ok = false;
+        }
+        ok = cudaStreamEndCapture(c.stream, &graph) == cudaSuccess && ok && graph != nullptr;
+        ok = ok && cudaGraphInstantiate(&r->exec, graph, 0) == cudaSuccess;
+        if (graph) cudaGraphDestroy(graph);
+        r->launches = c.launches - before;
+        c.launches = before;
+        if (!ok) {   // nothing of a failed recording has run
+            cudaGetLastError();
+            r->exec = nullptr;
+            r->unusable = true;
+        }
+    }
+    if (!r->exec) {
+        queue(s);
+        return;
+    }
+    FDK_CUDA(cudaGraphLaunch(r->exec, s));
+    c.launches += r->launches;
+}
+
+// Whether memory of the caller is page-locked, so that a copy from it is one DMA.
+static bool is_page_locked(const void* p) {
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return a.type == cudaMemoryTypeHost || a.type == cudaMemoryTypeManaged;
 }
 
 void Engine::run_block(DeviceCtx& c, const Plan& p, const std::vector<int64_t>& ids, const float* const* in_ptrs, float* const* out_ptrs,
@@ -1135,7 +1246,10 @@ void Engine::run_block(DeviceCtx& c, const Plan& p, const std::vector<int64_t>& 
     for (size_t o = 0; o < n_out; ++o) { out_e[o] = p.tensors[(size_t)p.outputs[o]].shape.volume(); out_total += round_up64(out_e[o], 64); }
     int dev_index = 0;
     for (size_t i = 0; i < ctx_.size(); ++i) if (ctx_[i].get() == &c) dev_index = (int)i;
-    const int64_t maxB = max_batch_for(p.in_shapes, dev_index);
+    // Largest batch: asking the driver for the free memory costs up to a millisecond, so it is asked only when the buffers
+    // have to grow.
+    int64_t maxB = std::min<int64_t>((int64_t)ids.size(), opt_.max_batch > 0 ? opt_.max_batch : 8192);
+    if (std::max<int64_t>(p.arena_elems, 64) * maxB > c.arena_elems || maxB * in_total > c.in_stage_elems) maxB = max_batch_for(p.in_shapes, dev_index);
     order_after_last_use(c, c.stream);
     for (size_t start = 0; start < ids.size(); start += (size_t)maxB) {
         const int64_t nb = (int64_t)std::min<size_t>((size_t)maxB, ids.size() - start);
@@ -1228,7 +1342,6 @@ void Engine::run_block(DeviceCtx& c, const Plan& p, const std::vector<int64_t>& 
             // done, which would hold the host back from queueing the next chunk.
             direct[o] = (contiguous && n_chunks == 1) ? 1 : 0;
         }
-        FDK_CUDA(cudaMemsetAsync(c.d_err, 0, sizeof(int), c.stream));
         int64_t off = 0;                       // running offset into the input staging buffers (floats)
         std::vector<int64_t> ooffs(n_out);     // offsets of the outputs in h_out: [output][sample] over the whole block
         {
@@ -1240,38 +1353,55 @@ void Engine::run_block(DeviceCtx& c, const Plan& p, const std::vector<int64_t>& 
                 const int64_t k0 = bounds[(size_t)ch], k1 = bounds[(size_t)ch + 1], cnb = k1 - k0;
                 if (cnb == 0) continue;
                 cudaStream_t cs = n_chunks > 1 ? c.copy_stream : c.stream;
+                // A block of a few kilobytes goes through page-locked memory that the first kernel reads itself.
+                const bool tiny = n_chunks == 1 && in_bytes <= (64 << 10);
                 std::vector<const float*> d_in(n_in);
+                std::vector<int64_t> at(n_in);   // offset of every input in the staging buffers
                 for (size_t i = 0; i < n_in; ++i) {
+                    at[i] = off;
                     d_in[i] = c.in_stage + off;
                     auto sample_ptr = [&](int64_t k) { return reinterpret_cast<const char*>(in_ptrs[(size_t)ids[start + (size_t)(k0 + k)] * n_in + i]); };
                     const char* first = sample_ptr(0);
+                    const size_t sample_bytes = esz * (size_t)in_e[i], n_bytes = sample_bytes * (size_t)cnb;
                     bool contiguous = true;  // the samples lie back to back in the caller's memory (a batch array)
-                    for (int64_t k = 1; k < cnb && contiguous; ++k) contiguous = sample_ptr(k) == first + (size_t)(k * in_e[i]) * esz;
-                    const size_t n_bytes = esz * (size_t)(cnb * in_e[i]);
+                    for (int64_t k = 1; k < cnb && contiguous; ++k) contiguous = sample_ptr(k) == first + (size_t)k * sample_bytes;
                     // where the copy lands: the float staging itself, or (byte inputs) the byte staging at the same offset
-                    void* d_dst = bytes ? (void*)(c.byte_stage + off) : (void*)(c.in_stage + off);
-                    if (contiguous) {
-                        // straight from the caller's buffer (a true DMA if it is pinned; the driver stages pageable memory)
-                        FDK_CUDA(cudaMemcpyAsync(d_dst, first, n_bytes, cudaMemcpyHostToDevice, cs));
-                        count_transfer(true, n_bytes);
-                    } else {
-                        // gather the samples into the pinned staging buffer, with a few threads when there is much to move
-                        char* dst = reinterpret_cast<char*>(c.h_in) + (size_t)off * esz;
-                        const int n_thr = n_bytes > (size_t)(8 << 20) ? (int)std::min<int64_t>(8, cnb) : 1;
-                        auto gather = [&](int64_t a0, int64_t a1) {
-                            for (int64_t k = a0; k < a1; ++k) std::memcpy(dst + (size_t)(k * in_e[i]) * esz, sample_ptr(k), esz * (size_t)in_e[i]);
-                        };
-                        if (n_thr == 1) {
-                            gather(0, cnb);
-                        } else {
-                            std::vector<std::thread> thr;
-                            for (int t = 0; t < n_thr; ++t) thr.emplace_back(gather, cnb * t / n_thr, cnb * (t + 1) / n_thr);
-                            for (auto& t : thr) t.join();
+                    char* d_dst = bytes ? reinterpret_cast<char*>(c.byte_stage + off) : reinterpret_cast<char*>(c.in_stage + off);
+                    char* h_dst = reinterpret_cast<char*>(c.h_in) + (size_t)off * esz;
+                    auto gather = [&](size_t b0, size_t b1) {   // bytes [b0, b1) of the input into page-locked memory
+                        if (contiguous) {
+                            std::memcpy(h_dst + b0, first + b0, b1 - b0);
+                            return;
                         }
-                        FDK_CUDA(cudaMemcpyAsync(d_dst, dst, n_bytes, cudaMemcpyHostToDevice, cs));
-                        count_transfer(true, n_bytes);
+                        for (size_t b = b0; b < b1;) {
+                            const size_t k = b / sample_bytes, in_sample = b - k * sample_bytes, n = std::min(sample_bytes - in_sample, b1 - b);
+                            std::memcpy(h_dst + b, sample_ptr((int64_t)k) + in_sample, n);
+                            b += n;
+                        }
+                    };
+                    if (n_bytes == 0) {
+                    } else if (tiny) {
+                        gather(0, n_bytes);
+                    } else if (contiguous && is_page_locked(first)) {
+                        FDK_CUDA(cudaMemcpyAsync(d_dst, first, n_bytes, cudaMemcpyHostToDevice, cs));
+                    } else {
+                        // Pageable or scattered samples: copied by several threads into page-locked memory, piece by piece, the
+                        // bus carrying one piece while the next is copied (the driver's own staging is one thread and waits).
+                        const size_t piece = (size_t)2 << 20;
+                        for (size_t b0 = 0; b0 < n_bytes; b0 += piece) {
+                            const size_t b1 = std::min(n_bytes, b0 + piece);
+                            if (b1 - b0 < ((size_t)256 << 10)) gather(b0, b1);
+                            else
+                                CopyPool::instance().run([&](int part, int parts) {
+                                    const size_t share = ((b1 - b0) / (size_t)parts + 4095) / 4096 * 4096;
+                                    const size_t p0 = std::min(b1, b0 + share * (size_t)part), p1 = part == parts - 1 ? b1 : std::min(b1, p0 + share);
+                                    if (p0 < p1) gather(p0, p1);
+                                });
+                            FDK_CUDA(cudaMemcpyAsync(d_dst + b0, h_dst + b0, b1 - b0, cudaMemcpyHostToDevice, cs));
+                        }
                     }
-                    if (bytes) launch_bytes_to_float(c.byte_stage + off, c.in_stage + off, cnb * in_e[i], bytes->low, bytes->high, cs);
+                    if (n_bytes > 0) count_transfer(true, n_bytes);
+                    if (bytes && n_chunks > 1) launch_bytes_to_float(c.byte_stage + off, c.in_stage + off, cnb * in_e[i], bytes->low, bytes->high, cs);
                     off += round_up64(cnb * in_e[i], 64);
                 }
                 if (n_chunks > 1) {
@@ -1279,29 +1409,56 @@ void Engine::run_block(DeviceCtx& c, const Plan& p, const std::vector<int64_t>& 
                     FDK_CUDA(cudaEventRecord(landed[(size_t)ch], cs));
                     FDK_CUDA(cudaStreamWaitEvent(c.stream, landed[(size_t)ch], 0));
                 }
-                execute(c, p, cnb, d_in.data(), c.stream);
-                // results of the chunk leave the arena before the next chunk overwrites it (same stream)
+                // a small result leaves with the kernel that also hands over the status words
+                const bool last = ch + 1 == n_chunks || bounds[(size_t)ch + 1] == nb;
+                const bool small_out = n_chunks == 1 && n_out == 1 && nb * out_e[0] <= 16384;
+                auto queue = [&](cudaStream_t on) {
+                    for (size_t i = 0; i < n_in; ++i) {
+                        const int64_t n = cnb * in_e[i];
+                        const void* host = reinterpret_cast<const char*>(c.h_in) + (size_t)at[i] * esz;
+                        if (tiny && bytes) launch_bytes_to_float(static_cast<const uint8_t*>(host), c.in_stage + at[i], n, bytes->low, bytes->high, on);
+                        else if (tiny) launch_fetch_host(host, c.in_stage + at[i], n * (int64_t)sizeof(float), on);
+                        else if (bytes && n_chunks == 1) launch_bytes_to_float(c.byte_stage + at[i], c.in_stage + at[i], n, bytes->low, bytes->high, on);
+                    }
+                    execute(c, p, cnb, d_in.data(), on, nullptr, nullptr, nullptr, nullptr, c.d_err + 1);
+                    // results of the chunk leave the arena before the next chunk overwrites it (same stream)
+                    for (size_t o = 0; o < n_out; ++o) {
+                        const BufferInfo& b = p.buffers[(size_t)p.tensors[(size_t)p.outputs[o]].buf];
+                        const float* src = b.ext_input >= 0 ? d_in[(size_t)b.ext_input] : c.arena + b.offset * cnb;
+                        if (small_out) {
+                            launch_export_host(src, c.h_out + ooffs[o], cnb * out_e[o], c.d_err + 1, c.status, c.h_err + 1, on);
+                            continue;
+                        }
+                        float* dst = direct[o] ? out_ptrs[(size_t)ids[start] * n_out + o] + k0 * out_e[o] : c.h_out + ooffs[o] + k0 * out_e[o];
+                        FDK_CUDA(cudaMemcpyAsync(dst, src, sizeof(float) * (size_t)(cnb * out_e[o]), cudaMemcpyDeviceToHost, on));
+                    }
+                    if (last && !small_out) launch_export_host(nullptr, nullptr, 0, c.d_err + 1, c.status, c.h_err + 1, on);
+                };
                 for (size_t o = 0; o < n_out; ++o) {
-                    const TensorInfo& t = p.tensors[(size_t)p.outputs[o]];
-                    const BufferInfo& b = p.buffers[(size_t)t.buf];
-                    const float* src = b.ext_input >= 0 ? d_in[(size_t)b.ext_input] : c.arena + b.offset * cnb;
-                    float* dst = direct[o] ? out_ptrs[(size_t)ids[start] * n_out + o] + k0 * out_e[o] : c.h_out + ooffs[o] + k0 * out_e[o];
-                    FDK_CUDA(cudaMemcpyAsync(dst, src, sizeof(float) * (size_t)(cnb * out_e[o]), cudaMemcpyDeviceToHost, c.stream));
+                    if (small_out) direct[o] = 0;
                     count_transfer(false, sizeof(float) * (size_t)(cnb * out_e[o]));
                 }
+                bool same_addresses = n_chunks == 1;   // a result that goes straight into the caller's memory has a new address every time
+                for (size_t o = 0; o < n_out; ++o) same_addresses = same_addresses && !direct[o];
+                if (same_addresses) {
+                    std::vector<const void*> where = {c.in_stage, c.h_in, c.h_out, bytes ? (const void*)c.byte_stage : nullptr, tiny ? (const void*)c.h_err : nullptr};
+                    replay(c, p, cnb, std::move(where), bytes ? bytes->low : 0.f, bytes ? bytes->high : 0.f, c.stream, queue);
+                } else {
+                    queue(c.stream);
+                }
             }
-            FDK_CUDA(cudaMemcpyAsync(c.h_err, c.d_err, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
             FDK_CUDA(cudaStreamSynchronize(c.stream));
             c.busy_valid = false;  // this stream waited for the last user and has finished itself: nothing is in flight
         } catch (...) {
             cudaStreamSynchronize(c.copy_stream);
             cudaStreamSynchronize(c.stream);
+            cudaMemset(c.d_err + 1, 0, sizeof(int));   // (the kernel that clears it may not have been launched)
             for (cudaEvent_t e : landed) if (e) cudaEventDestroy(e);
             throw;
         }
         for (cudaEvent_t e : landed) if (e) cudaEventDestroy(e);
-        if (*c.h_err != 0) raise(input_error_text(*c.h_err));
-        const int st = gemm_tc_take_status(c.stream);
+        if (c.h_err[1] != 0) raise(input_error_text(c.h_err[1]));
+        const int st = (c.h_err[2] | c.h_err[3] | c.h_err[4]) != 0 ? gemm_tc_take_status(c.stream) : 0;   // prints what gave up, clears the words
         if (st != 0) raise("tensor-core contraction kernel gave up waiting on a barrier (status " + std::to_string(st) + ")");
         for (size_t o = 0; o < n_out; ++o) {
             if (direct[o]) continue;
@@ -1317,12 +1474,17 @@ void Engine::predict_multi(int64_t n_samples, const float* const* in_ptrs, const
     // group by shape signature, keeping input order inside each group
     std::vector<std::pair<std::string, std::vector<int64_t>>> groups;
     std::map<std::string, size_t> gi;
+    size_t last_group = 0;
     for (int64_t sidx = 0; sidx < n_samples; ++sidx) {
-        std::vector<TShape> sh(in_shapes + sidx * (int64_t)n_in, in_shapes + (sidx + 1) * (int64_t)n_in);
-        const std::string key = signature(sh);
+        const TShape* shapes = in_shapes + sidx * (int64_t)n_in;
+        if (sidx > 0 && std::equal(shapes, shapes + n_in, shapes - n_in)) {   // as the sample before: the usual case
+            groups[last_group].second.push_back(sidx);
+            continue;
+        }
+        const std::string key = signature(std::vector<TShape>(shapes, shapes + n_in));
         auto it = gi.find(key);
-        if (it == gi.end()) { gi[key] = groups.size(); groups.emplace_back(key, std::vector<int64_t>{sidx}); }
-        else groups[it->second].second.push_back(sidx);
+        if (it == gi.end()) { last_group = groups.size(); gi[key] = last_group; groups.emplace_back(key, std::vector<int64_t>{sidx}); }
+        else { last_group = it->second; groups[last_group].second.push_back(sidx); }
     }
     for (auto& gr : groups) {
         const std::vector<int64_t>& ids = gr.second;

@@ -73,6 +73,19 @@ struct DeviceWeights {
     std::vector<int64_t> small_offset;  // TF32 low halves or -1
 };
 
+// The launches of one call, recorded as a CUDA graph: everything that fixes them is in the key (the plan, the batch and every
+// address the launches hold).
+struct RecordedCall {
+    const Plan* plan = nullptr;
+    int64_t batch = 0;
+    std::vector<const void*> where;    // caller's buffers or staging buffers, arena, workspace
+    float low = 0.f, high = 0.f;
+    cudaGraphExec_t exec = nullptr;
+    int64_t launches = 0;
+    uint64_t last_use = 0;
+    bool unusable = false;             // could not be recorded: launch directly
+};
+
 struct DeviceCtx {
     uint8_t* byte_stage = nullptr;   // device staging for byte inputs
     int64_t byte_stage_bytes = 0;
@@ -93,8 +106,13 @@ struct DeviceCtx {
     int64_t h_out_elems = 0;
     float* workspace = nullptr;    // partial tiles of split-K products
     int64_t workspace_elems = 0;
-    int* d_err = nullptr;          // device error flag (embedding range)
-    int* h_err = nullptr;          // pinned
+    // Input checks on the device (embedding range, ...): [0] for calls that leave work in flight (read by fdk_model_sync),
+    // [1] for host calls, cleared by the kernel that ends each of them.
+    int* d_err = nullptr;
+    int* h_err = nullptr;          // page-locked: [0] as above, [1 .. 4] the words a host call ends with (launch_export_host)
+    const int* status[3] = {nullptr, nullptr, nullptr};   // device addresses of the contraction and tile kernels' status words
+    std::vector<RecordedCall> calls;   // see Engine::replay
+    uint64_t call_clock = 0;
     std::mutex mu;                 // held while a call queues its work on this device
     // Order between calls that use the arena / workspace from different streams: the last use recorded `busy` on
     // `busy_stream`; the next use on another stream waits for it (Engine::order_after_last_use / mark_use).
@@ -205,10 +223,15 @@ public:
 private:
     std::shared_ptr<Plan> get_plan(const std::vector<TShape>& in_shapes);
     std::shared_ptr<Plan> compile(const std::vector<TShape>& in_shapes);
-    // wanted (optional, per plan output): 0 = the caller does not read this output, so it need not be computed
+    // wanted (optional, per plan output): 0 = the caller does not read this output, so it need not be computed.
+    // d_out (optional, per plan output): where the caller wants it; set entries have to be copied there afterwards only if
+    // `bound_output` says that the producing kernel cannot write there itself.  err: flag of the device-side input checks.
     void execute(DeviceCtx& c, const Plan& p, int64_t B, const float* const* d_in, cudaStream_t s, std::string* profile = nullptr,
-                 const KvCache* kv = nullptr, const std::vector<char>* wanted = nullptr);
+                 const KvCache* kv = nullptr, const std::vector<char>* wanted = nullptr, float* const* d_out = nullptr, int* err = nullptr);
     void ensure_arena(DeviceCtx& c, int64_t elems);
+    // Runs `queue(stream)` or replays what it launched before (see RecordedCall); call with c.mu held.
+    template <typename F>
+    void replay(DeviceCtx& c, const Plan& p, int64_t batch, std::vector<const void*> where, float low, float high, cudaStream_t s, F&& queue);
     void run_block(DeviceCtx& c, const Plan& p, const std::vector<int64_t>& sample_ids, const float* const* in_ptrs,
                    float* const* out_ptrs, const ByteScale* bytes = nullptr);
     void upload_weights(DeviceCtx& c);

@@ -2003,7 +2003,37 @@ __global__ void publish_position_kernel(const float* __restrict__ tokens, int n,
     }
     __threadfence_system();
 }
+// Values of a small host call in and out: the caller's samples lie in page-locked memory that the kernel reads over the
+// bus itself, and the results and status words go back the same way.  A copy engine would cost a hop of several
+// microseconds each way for a few kilobytes.
+__global__ void __launch_bounds__(256) fetch_host_kernel(const uint4* __restrict__ in, uint4* __restrict__ out, int n16) {
+    pdl_launch_dependents();
+    pdl_wait();
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n16; i += gridDim.x * blockDim.x) out[i] = in[i];
+}
+__global__ void __launch_bounds__(512) export_host_kernel(const float* __restrict__ src, float* __restrict__ host, int n, int* err,
+                                                          const int* s0, const int* s1, const int* s2, int* __restrict__ host_words) {
+    pdl_launch_dependents();
+    pdl_wait();
+    for (int i = threadIdx.x; i < n; i += blockDim.x) host[i] = __ldcg(src + i);
+    if (threadIdx.x == 0) {
+        host_words[0] = __ldcg(err);
+        host_words[1] = __ldcg(s0);
+        host_words[2] = __ldcg(s1);
+        host_words[3] = __ldcg(s2);
+        *err = 0;
+    }
+    __threadfence_system();
+}
 }  // namespace
+void launch_fetch_host(const void* host, void* out, int64_t bytes, cudaStream_t s) {
+    const int n16 = (int)((bytes + 15) / 16);
+    if (n16 <= 0) return;
+    launch_pdl(fetch_host_kernel, dim3((unsigned)((n16 + 255) / 256)), dim3(256), 0, s, static_cast<const uint4*>(host), static_cast<uint4*>(out), n16);
+}
+void launch_export_host(const float* src, float* host, int64_t n, int* err, const int* const (&status)[3], int* host_words, cudaStream_t s) {
+    launch_pdl(export_host_kernel, dim3(1), dim3(512), 0, s, src, host, (int)n, err, status[0], status[1], status[2], host_words);
+}
 void launch_publish_position(const float* tokens, int n, const int* status_a, const int* status_b, float* host_tokens, int* host_status,
                              cudaStream_t s) {
     launch_pdl(publish_position_kernel, dim3(1), dim3(128), 0, s, tokens, n, status_a, status_b, host_tokens, host_status);

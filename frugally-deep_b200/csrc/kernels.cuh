@@ -262,9 +262,14 @@ void launch_argmax_rows(const float* in, float* out, int64_t rows, int n, cudaSt
 // synchronised the host reads them without any further call.  host_status receives {status_a, status_b}.
 void launch_publish_position(const float* tokens, int n, const int* status_a, const int* status_b, float* host_tokens, int* host_status,
                              cudaStream_t s);
+// A small host call: reads `bytes` (rounded up to 16; both buffers 16-byte aligned) of page-locked host memory into `out`.
+void launch_fetch_host(const void* host, void* out, int64_t bytes, cudaStream_t s);
+// End of a host call: n floats into page-locked host memory, host_words = {*err, three status words}; *err is cleared.
+void launch_export_host(const float* src, float* host, int64_t n, int* err, const int* const (&status)[3], int* host_words, cudaStream_t s);
 // Device addresses (on the current device) of the status words read by gemm_tc_take_status.
 const int* gemm_tc_status_address();
 const int* gemm_rows_status_address();
+const int* dwconv_tiles_status_address();
 // out = in * f (Average layer: sum * (1 / n), tensor.hpp:886-891)
 void launch_scale(const float* in, float* out, int64_t n, float f, cudaStream_t s);
 

@@ -121,6 +121,10 @@ def _dims5(shape: Sequence[int]) -> List[int]:
     return [1] * (5 - len(shape)) + [int(s) for s in shape]
 
 
+def _address(a: np.ndarray) -> int:
+    return a.__array_interface__["data"][0]
+
+
 FLAG_NO_TENSOR_CORES = 1
 FLAG_SKINNY_PRODUCTS = 2
 FLAG_FUSED_CELLS = 4
@@ -131,6 +135,7 @@ class Model:
 
     def __init__(self, handle):
         self._h = handle
+        self._shape_cache = {}
         L = load_library()
         self.n_inputs = L.fdk_model_num_inputs(handle)
         self.n_outputs = L.fdk_model_num_outputs(handle)
@@ -197,63 +202,68 @@ class Model:
     def predict_multi(self, samples: Sequence[Sequence[np.ndarray]], bytes_range: Optional[Sequence[float]] = None) -> List[List[np.ndarray]]:
         """model::predict_multi (model.hpp:31-42): samples[s][i] is input i of sample s (host arrays).  With
         bytes_range = (low, high) the inputs are uint8 arrays scaled into that range on the GPU."""
-        L = load_library()
         ns = len(samples)
         if ns == 0:
             return []
         n_in, n_out = self.n_inputs, self.n_outputs
+        dtype = np.uint8 if bytes_range is not None else np.float32
         arrs = []
         for s in samples:
             if len(s) != n_in:
                 raise FdeepError(f"Invalid number of input tensors for this model: {n_in} required but {len(s)} provided")
-            arrs.append([np.ascontiguousarray(a, dtype=np.uint8 if bytes_range is not None else np.float32) for a in s])
-        shape_cache = {}
-        outs = []
+            arrs.append([np.ascontiguousarray(a, dtype=dtype) for a in s])
+        outs, dims, ranks = [], [], []
         for s in arrs:
-            key = tuple(a.shape for a in s)
-            if key not in shape_cache:
-                shape_cache[key] = self.infer_shapes([a.shape for a in s])
-            outs.append([np.empty(sh, dtype=np.float32) for sh in shape_cache[key]])
-        in_ptrs = (C.c_void_p * (ns * n_in))(*[a.ctypes.data for s in arrs for a in s])
-        dims = (C.c_int64 * (5 * ns * n_in))(*[d for s in arrs for a in s for d in _dims5(a.shape)])
-        ranks = (C.c_int * (ns * n_in))(*[a.ndim for s in arrs for a in s])
-        out_ptrs = (C.c_void_p * (ns * n_out))(*[o.ctypes.data for s in outs for o in s])
+            out_shapes, d, r = self._shapes(tuple([a.shape for a in s]))
+            outs.append([np.empty(sh, dtype=np.float32) for sh in out_shapes])
+            dims += d
+            ranks += r
+        in_ptrs = (C.c_void_p * (ns * n_in))(*[_address(a) for s in arrs for a in s])
+        out_ptrs = (C.c_void_p * (ns * n_out))(*[_address(o) for s in outs for o in s])
+        self._predict_multi(ns, in_ptrs, (C.c_int64 * len(dims))(*dims), (C.c_int * len(ranks))(*ranks), out_ptrs, bytes_range)
+        return outs
+
+    def _shapes(self, in_shapes):
+        """(output shapes, input dims as fdk_* calls take them, input ranks) for one sample's input shapes; looked up once per
+        kind of sample."""
+        known = self._shape_cache.get(in_shapes)
+        if known is None:
+            known = (self.infer_shapes(in_shapes), [d for s in in_shapes for d in _dims5(s)], [len(s) for s in in_shapes])
+            if len(self._shape_cache) >= 4096:
+                self._shape_cache.clear()
+            self._shape_cache[in_shapes] = known
+        return known
+
+    def _predict_multi(self, ns, in_ptrs, dims, ranks, out_ptrs, bytes_range):
+        L = load_library()
         if bytes_range is not None:
             _check(L.fdk_model_predict_multi_u8(self._h, ns, in_ptrs, dims, ranks, float(bytes_range[0]), float(bytes_range[1]), out_ptrs))
         else:
             _check(L.fdk_model_predict_multi(self._h, ns, in_ptrs, dims, ranks, out_ptrs))
-        return outs
 
     def predict_batch(self, inputs: Sequence[np.ndarray], bytes_range: Optional[Sequence[float]] = None) -> List[np.ndarray]:
         """Convenience for equally shaped samples: inputs[i] has shape (batch, ...); one call of
         predict_multi on views of the batch arrays, outputs stacked the same way.  With bytes_range =
         (low, high) the inputs are uint8 arrays that are scaled into that range on the GPU
         (tensor_from_bytes, tensor.hpp:1230-1245)."""
-        L = load_library()
         n_in, n_out = self.n_inputs, self.n_outputs
         arrs = [np.ascontiguousarray(a, dtype=np.uint8 if bytes_range is not None else np.float32) for a in inputs]
         ns = arrs[0].shape[0]
-        out_shapes = self.infer_shapes([a.shape[1:] for a in arrs])
+        if len(arrs) != n_in:
+            raise FdeepError(f"Invalid number of input tensors for this model: {n_in} required but {len(arrs)} provided")
+        out_shapes, one, one_rank = self._shapes(tuple([a.shape[1:] for a in arrs]))
         outs = [np.empty([ns] + list(sh), dtype=np.float32) for sh in out_shapes]
-        in_ptrs = (C.c_void_p * (ns * n_in))()
-        out_ptrs = (C.c_void_p * (ns * n_out))()
-        for i, a in enumerate(arrs):
-            stride = a.strides[0] if ns > 0 else 0
-            base = a.ctypes.data
-            for s in range(ns):
-                in_ptrs[s * n_in + i] = base + s * stride
-        for o, a in enumerate(outs):
-            stride = a.strides[0] if ns > 0 else 0
-            base = a.ctypes.data
-            for s in range(ns):
-                out_ptrs[s * n_out + o] = base + s * stride
-        one = [d for a in arrs for d in _dims5(a.shape[1:])]
-        dims = (C.c_int64 * (5 * ns * n_in))(*(one * ns))
-        ranks = (C.c_int * (ns * n_in))(*([a.ndim - 1 for a in arrs] * ns))
-        if bytes_range is not None:
-            _check(L.fdk_model_predict_multi_u8(self._h, ns, in_ptrs, dims, ranks, float(bytes_range[0]), float(bytes_range[1]), out_ptrs))
-        else:
-            _check(L.fdk_model_predict_multi(self._h, ns, in_ptrs, dims, ranks, out_ptrs))
+        if ns == 0:
+            return outs
+        # one array of addresses per call, written without a Python loop over the samples
+        row = np.arange(ns, dtype=np.uint64)[:, None]
+        in_ptrs = np.array([_address(a) for a in arrs], np.uint64) + row * np.array([a.strides[0] for a in arrs], np.uint64)
+        out_ptrs = np.array([_address(a) for a in outs], np.uint64) + row * np.array([a.strides[0] for a in outs], np.uint64)
+        dims = np.tile(np.array(one, np.int64), ns)
+        ranks = np.tile(np.array(one_rank, np.intc), ns)
+        vpp = C.POINTER(C.c_void_p)
+        self._predict_multi(ns, in_ptrs.ctypes.data_as(vpp), dims.ctypes.data_as(C.POINTER(C.c_int64)), ranks.ctypes.data_as(C.POINTER(C.c_int)),
+                            out_ptrs.ctypes.data_as(vpp), bytes_range)
         return outs
 
     def predict_batch_device(self, d_in_ptrs: Sequence[int], in_shapes: Sequence[Sequence[int]], batch: int,

@@ -340,6 +340,10 @@ struct Exec {
             gemm_skinny_plan(N, K, slices, kps, ws, M);
             ensure_workspace(ws);
             launch_gemm_skinny(A, lda, W, ldw, C, ldc, M, N, K, e, c.workspace, s, use_tc);
+        } else if (float* parts = tc ? group_sums(gemm_tc_parts_floats(M, N, K)) : nullptr) {
+            launch_gemm_tc_parts(A, lda, c.w.base + c.w.big_offset[(size_t)w_id] + w_off, c.w.base + c.w.small_offset[(size_t)w_id] + w_off, ldw, C,
+                                 ldc, M, N, K, e, parts, s);
+            c.launches++;
         } else if (tc) {
             launch_gemm_tc(A, lda, c.w.base + c.w.big_offset[(size_t)w_id] + w_off, c.w.base + c.w.small_offset[(size_t)w_id] + w_off, ldw, C, ldc, M,
                            N, K, e, s);
@@ -356,14 +360,37 @@ struct Exec {
     // The workspace may move when it grows (a recorded graph that holds the old address must be recorded again: the
     // decode session compares addresses before every replay).
     void ensure_workspace(int64_t ws) {
-        if (ws <= c.workspace_elems) return;
+        ensure(try_workspace(ws), "device workspace allocation of " + std::to_string(ws * 4) + " bytes failed");
+    }
+    // Group sums of products of few rows (gemm_tc.cu) live behind the arrival counters, one part per chain of time steps
+    // (their products run side by side).  Null: not wanted (floats = 0), or no memory for it, and the product runs whole.
+    static constexpr int64_t WORKSPACE_COUNTERS = 1024;
+    int chain = 0;               // which part this product uses
+    int64_t chain_floats = 0;    // size of the first chain's part while two chains run (-1: no memory for both), else 0
+    float* group_sums(int64_t floats) {
+        if (floats <= 0 || chain_floats < 0) return nullptr;
+        const int64_t first = WORKSPACE_COUNTERS + (chain ? chain_floats : 0);
+        if (!try_workspace(first + floats)) return nullptr;
+        return c.workspace + first;
+    }
+    bool try_workspace(int64_t ws) {
+        if (ws <= c.workspace_elems) return true;
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        FDK_CUDA(cudaStreamIsCapturing(s, &cap));
+        if (cap != cudaStreamCaptureStatusNone) return false;   // nothing may be allocated here
         FDK_CUDA(cudaStreamSynchronize(s));
+        if (c.aux_stream) FDK_CUDA(cudaStreamSynchronize(c.aux_stream));
         if (c.busy_valid) FDK_CUDA(cudaEventSynchronize(c.busy));
         if (c.workspace) FDK_CUDA(cudaFree(c.workspace));
         c.workspace = nullptr; c.workspace_elems = 0;
-        FDK_CUDA(cudaMalloc(&c.workspace, sizeof(float) * (size_t)ws));
+        if (cudaMalloc(&c.workspace, sizeof(float) * (size_t)ws) != cudaSuccess) {
+            cudaGetLastError();
+            c.workspace = nullptr;
+            return false;
+        }
         FDK_CUDA(cudaMemset(c.workspace, 0, sizeof(float) * (size_t)ws));  // the arrival counters start at zero (synchronous)
         c.workspace_elems = ws;
+        return true;
     }
     // Query, key and value projections of one attention block on the same rows: one launch of the skinny kernel when
     // all three qualify for it (same shape, bias-only epilogues).  Returns false when nothing was launched.
@@ -777,8 +804,14 @@ struct Exec {
                 r = Rec{"gemm", o.layer->name, "tc", nullptr, nullptr, 2.0 * (double)M * o.N * o.K, M, o.N, o.K};
                 rec_begin(r);
             }
-            launch_conv_tc(in, g, c.w.base + c.w.big_offset[(size_t)w_id], c.w.base + c.w.small_offset[(size_t)w_id], ldw,
-                           tptr(o.out[0]), o.N, o.N, e, s);
+            if (float* parts = group_sums(conv_tc_parts_floats(g, o.N))) {
+                launch_conv_tc_parts(in, g, c.w.base + c.w.big_offset[(size_t)w_id], c.w.base + c.w.small_offset[(size_t)w_id], ldw, tptr(o.out[0]),
+                                     o.N, o.N, e, parts, s);
+                c.launches++;
+            } else {
+                launch_conv_tc(in, g, c.w.base + c.w.big_offset[(size_t)w_id], c.w.base + c.w.small_offset[(size_t)w_id], ldw, tptr(o.out[0]), o.N, o.N, e,
+                               s);
+            }
             if (prof) {
                 FDK_CUDA(cudaEventRecord(r.b, s));
                 prof->push_back(r);
@@ -859,6 +892,13 @@ struct Exec {
         FDK_CUDA(cudaMemsetAsync(c2, 0, sizeof(float) * (size_t)(B * U), s));
         float* hc = h;
         float* hn = c2;  // SimpleRNN ping-pong
+        // LSTM on few rows: the recurrent product leaves its group sums and the cell kernel adds them (same results)
+        auto step_sums = [&](int64_t nb) -> float* {
+            if (o.kind != OP_LSTM || !use_tc || use_skinny || L.act_main.kind != ACT_TANH || L.act_rec.kind != ACT_SIGMOID || nb * U > 0x1fffffffLL ||
+                c.w.big_offset[(size_t)L.w_rec] < 0 || !gemm_tc_supported(nb, gu, U, U, L.kdim, h, wptr(L.w_rec)))
+                return nullptr;
+            return group_sums(gemm_tc_parts_floats(nb, gu, U));
+        };
         // The time steps of rows [r0, r0 + nb) of the batch, queued on the executor's current stream.  h_in / h_out: where
         // this step reads and leaves the state ([B][U]; the same buffer except for SimpleRNN and the fused LSTM step).
         auto rows_step = [&](int64_t r0, int64_t nb, int64_t t, float* o_ptr, int64_t o_stride, float* h_in, float* h_out) {
@@ -881,6 +921,21 @@ struct Exec {
                     prof->push_back(r);
                 }
                 c.launches++;
+            } else if (float* parts = step_sums(nb)) {
+                Rec r;
+                if (prof) {
+                    r = Rec{"gemm", L.name, "tc sums", nullptr, nullptr, 2.0 * (double)nb * gu * U, nb, gu, U};
+                    rec_begin(r);
+                }
+                const int groups = launch_gemm_tc_group_sums(hr, U, c.w.base + c.w.big_offset[(size_t)L.w_rec], c.w.base + c.w.small_offset[(size_t)L.w_rec],
+                                                             L.kdim, nb, gu, U, parts, s);
+                if (prof) {
+                    FDK_CUDA(cudaEventRecord(r.b, s));
+                    prof->push_back(r);
+                }
+                c.launches += 2;
+                ensure(launch_lstm_cell_parts(parts, groups, xr, T * gu, cr, hr, outr, o_stride, nb, U, L.act_main, L.act_rec, s),
+                       "internal: the cell on group sums was not launched");
             } else if (o.kind == OP_LSTM) {
                 Epilogue e;
                 e.residual = xr;
@@ -921,6 +976,16 @@ struct Exec {
         // the batch they are computed in, so the split cannot change them.
         const bool two_chains = prof == nullptr && B >= 256 && c.aux_stream != nullptr && c.aux_stream != s;
         const int64_t first_rows = two_chains ? (B / 2 + 127) / 128 * 128 : B;
+        struct ChainParts {   // both chains' group sums, in place before the first launch
+            int64_t& floats;
+            ~ChainParts() { floats = 0; }
+        } chain_parts{chain_floats};
+        if (two_chains) {
+            auto most = [&](int64_t nb) { return std::max(gemm_tc_parts_floats(nb, gu, U), gemm_tc_parts_floats(nb, U, U)); };
+            chain_floats = std::max(most(first_rows), gemm_tc_parts_floats(first_rows, 2 * U, U));
+            const int64_t second = std::max(most(B - first_rows), gemm_tc_parts_floats(B - first_rows, 2 * U, U));
+            if (chain_floats + second > 0 && !try_workspace(WORKSPACE_COUNTERS + chain_floats + second)) chain_floats = -1;
+        }
         cudaStream_t main_stream = s;
         if (two_chains) {
             FDK_CUDA(cudaEventRecord(c.fork_event, main_stream));
@@ -938,12 +1003,15 @@ struct Exec {
                 rows_step(0, first_rows, t, o_ptr, o_stride, h_in, h_out);
                 if (two_chains) {
                     s = c.aux_stream;
+                    chain = 1;
                     rows_step(first_rows, B - first_rows, t, o_ptr, o_stride, h_in, h_out);
+                    chain = 0;
                     s = main_stream;
                 }
             } catch (...) {
                 // nothing of the second chain may still run when the caller's stream goes on (or the arena is reused)
                 s = main_stream;
+                chain = 0;
                 if (two_chains) cudaStreamSynchronize(c.aux_stream);
                 throw;
             }

@@ -40,7 +40,8 @@
 //     row coordinate beyond the image;
 //   * transposed convolutions (convolution.hpp:443-469), one launch per output phase: sub-filter, pad = -shift, and
 //     output pixels that lie sx * N, sy * Wo * N floats apart (the output and residual tensor maps carry the strides);
-//   * an LSTM time step (recurrent_ops.hpp:164-181) as the kernel instance CELL = true, whose epilogue forms the gate
+//   * a run of a tile's k blocks (instance TC_PARTS), whose group sums leave unadded;
+//   * an LSTM time step (recurrent_ops.hpp:164-181) as the kernel instance TC_CELL, whose epilogue forms the gate
 //     pre-activations in the staging buffers and finishes the cell instead of storing them.
 #include "kernels.cuh"
 #include "device_math.cuh"
@@ -121,6 +122,10 @@ constexpr int TC_THREADS = (TC_EPI_WARP0 + 8) * 32;
 constexpr int TC_REGS_LAUNCH = TC_TEAMS == 1 ? 128 : 96;
 constexpr int TC_REGS_CONTROL = TC_TEAMS == 1 ? 56 : 48, TC_REGS_CONVERT = 112, TC_REGS_EPILOGUE = TC_TEAMS == 1 ? 168 : 104;
 static_assert(128 * TC_REGS_CONTROL + 128 * TC_TEAMS * TC_REGS_CONVERT + 256 * TC_REGS_EPILOGUE <= TC_THREADS * TC_REGS_LAUNCH, "register budget");
+// Kernel instances: a whole product; an LSTM time step (the epilogue ends the cell); the group sums of a product whose
+// k blocks are spread over CTAs (see split_plan).
+constexpr int64_t SPLIT_MAX_FLOATS = 8 << 20;   // group sums of one product: at most 32 MB, a quarter of L2
+enum TcMode : int { TC_PRODUCT = 0, TC_CELL = 1, TC_PARTS = 2 };
 constexpr unsigned long long TC_WAIT_LIMIT_NS = 2000000000ull;  // 2 s: far beyond any legitimate wait
 
 __device__ int g_tc_status = 0;
@@ -249,6 +254,7 @@ struct TcParams {
     int tiles_w, tiles_h, tiles_n;
     int nbuf;                         // staging buffers per epilogue warp (1 or 2)
     int tma_epi;                      // 1: output (and residual) rows are 16-byte aligned: TMA epilogue
+    int runs, kb_run;                 // PARTS: runs per tile, k blocks per run (a multiple of TC_GROUP)
     EpiDev epi;
     // LSTM step (kernel instance with CELL = true): state tensors [B][cell_U]; cell_out may be null
     float* cell_c;
@@ -386,12 +392,13 @@ __device__ __forceinline__ void lstm_cell_row(const uint8_t* __restrict__ row0, 
     }
 }
 
-template <int BN, bool CELL>
+template <int BN, int MODE>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapWb,
                const __grid_constant__ CUtensorMap mapWs, const __grid_constant__ CUtensorMap mapC,
                const __grid_constant__ CUtensorMap mapR, TcParams prm) {
     using Cfg = TcCfg<BN>;
+    constexpr bool CELL = MODE == TC_CELL, PARTS = MODE == TC_PARTS;
     const int STAGES = prm.stages;      // W ring / A slots: 2..Cfg::STAGES
     const int A_STAGES = prm.a_stages;  // raw A ring: 2..Cfg::A_STAGES
     // The swizzled tiles need 1024-byte alignment; the kernel has no static shared memory, so the dynamic part
@@ -466,9 +473,14 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
     // tile indices fit 32 bits (checked by the host): 32-bit divisions keep the code small
     const uint32_t m_tiles = (uint32_t)prm.tiles_n * (uint32_t)prm.tiles_h * (uint32_t)prm.tiles_w;
     const int n_tiles = (prm.N + BN - 1) / BN;
-    const uint32_t tiles = m_tiles * (uint32_t)n_tiles;
+    // PARTS: a tile's k blocks are dealt out in runs of kb_run to `runs` work units; otherwise a unit is a tile
+    const uint32_t runs = PARTS ? (uint32_t)prm.runs : 1u;
+    const uint32_t units = m_tiles * (uint32_t)n_tiles * runs;
     const uint32_t tiles_wh = (uint32_t)prm.tiles_w * (uint32_t)prm.tiles_h;
-    const int k_blocks = prm.taps * prm.cchunks;
+    const int all_blocks = prm.taps * prm.cchunks;
+    const int kb_run = PARTS ? prm.kb_run : all_blocks;
+    auto unit_first = [&](uint32_t unit) { return PARTS ? (int)(unit % runs) * kb_run : 0; };                        // its first k block
+    auto unit_blocks = [&](uint32_t unit) { return PARTS ? min(kb_run, all_blocks - unit_first(unit)) : all_blocks; };  // how many it has
 
     auto a_ptr = [&](int s) { return base + (uint32_t)s * (uint32_t)Cfg::A_BYTES; };
     auto w_ptr = [&](int s) { return base + w_off + (uint32_t)s * (uint32_t)Cfg::W_BYTES; };
@@ -489,8 +501,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
         int stage = 0;
         uint32_t phase = 0;
         bool ok = true;
-        for (uint32_t tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
-            if (!a_role && prm.w_stationary && tile != blockIdx.x) break;  // the weights of the first tile serve all
+        for (uint32_t unit = blockIdx.x; unit < units && ok; unit += gridDim.x) {
+            if (!a_role && prm.w_stationary && unit != blockIdx.x) break;  // the weights of the first tile serve all
+            const uint32_t tile = unit / runs;
+            const int k_blocks = unit_blocks(unit);
             const uint32_t mt = tile / (uint32_t)n_tiles;
             const int n0 = (int)(tile % (uint32_t)n_tiles) * BN;
             const int tw = (int)(mt % (uint32_t)prm.tiles_w);
@@ -507,6 +521,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
                 b0 = sample * prm.Din;
             }
             int tap = 0, cc = 0, ky = 0, kx = 0, kz = 0;
+            if constexpr (PARTS) {   // (no 3-D walk in this form)
+                const int first = unit_first(unit);
+                tap = first / prm.cchunks;
+                cc = first - tap * prm.cchunks;
+                ky = tap / prm.kw;
+                kx = tap - ky * prm.kw;
+            }
             for (int kb = 0; kb < k_blocks; ++kb) {
                 if (!mbar_wait(a_role ? afree_bar(stage) : empty_bar(stage), phase ^ 1u, abort_flag, 1)) { ok = false; break; }
                 if (lane == 0) {
@@ -559,7 +580,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
         uint32_t phase = 0, set_phase = 0;
         uint32_t gg = 0;
         bool ok = true;
-        for (uint32_t tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
+        for (uint32_t unit = blockIdx.x; unit < units && ok; unit += gridDim.x) {
+            const int k_blocks = unit_blocks(unit);
             for (int kb = 0; kb < k_blocks; kb += TC_GROUP, ++gg) {
                 const int nb = k_blocks - kb < TC_GROUP ? k_blocks - kb : TC_GROUP;
                 const int s0 = stage;
@@ -684,16 +706,60 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
             }
         };
         bool res_ready = false;  // res_ahead: the current tile's residual blocks were requested one tile ago
-        if (res_ahead && blockIdx.x < tiles) {
+        if (res_ahead && blockIdx.x < units) {
             const TileGeom g0 = geom_of(blockIdx.x);
             if (g0.tma_tile && g0.box_in) {
                 if (lane == 0) request_residual(g0, 0);
                 res_ready = true;
             }
         }
-        for (uint32_t tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
+        for (uint32_t unit = blockIdx.x; unit < units && ok; unit += gridDim.x) {
+            const uint32_t tile = unit / runs;
+            const int k_blocks = unit_blocks(unit);
             const TileGeom g = geom_of(tile);
             const int n0 = g.n0;
+            if constexpr (PARTS) {
+                // ---- every group sum leaves as it is: parts[group][pixel][column]; sum_parts_kernel adds them up ----
+                const int first_group = unit_first(unit) / TC_GROUP;
+                for (int kb = 0; kb < k_blocks; kb += TC_GROUP) {
+                    if (!mbar_wait(tfull_bar(acc), acc_phase, abort_flag, 4)) { ok = false; break; }
+                    tc_fence_after();
+                    const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * BN + half * CPT);
+                    const int nsub = g.box_in ? g.nsub : 0;
+#pragma unroll 1
+                    for (int j = 0; j < nsub; ++j) {
+                        if (lane == 0) {
+                            if (nbuf >= 4) bulk_wait_read<3>();
+                            else if (nbuf == 2) bulk_wait_read<1>();
+                            else bulk_wait_read<0>();
+                        }
+                        __syncwarp();
+                        uint32_t r[32];
+                        tmem_ld32(taddr + 32u * (uint32_t)j, r);
+                        tmem_ld_wait();
+                        const uint32_t row_s = stg_addr + (uint32_t)(ring * Cfg::STG_BUF_BYTES + lane * 128);
+#pragma unroll
+                        for (int c = 0; c < 8; ++c)
+                            tc_sts4(row_s + (uint32_t)((c ^ (lane & 7)) << 4),
+                                    make_float4(__uint_as_float(r[4 * c]), __uint_as_float(r[4 * c + 1]), __uint_as_float(r[4 * c + 2]),
+                                                __uint_as_float(r[4 * c + 3])));
+                        fence_proxy_async();
+                        __syncwarp();
+                        if (lane == 0) {
+                            tma_store_5d(&mapC, stg_addr + (uint32_t)(ring * Cfg::STG_BUF_BYTES), n0 + 32 * j, g.qx, g.qy, g.qb,
+                                         first_group + kb / TC_GROUP);
+                            bulk_commit();
+                        }
+                        __syncwarp();
+                        ring = (ring + 1) & (nbuf - 1);
+                    }
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(tempty_bar(acc));
+                    if (++acc == SETS) { acc = 0; acc_phase ^= 1u; }
+                }
+                continue;
+            }
             if (g.tma_tile && n0 != prm_n0) {
                 __syncwarp();
                 for (int c = lane; c < CPT; c += 32) {
@@ -706,7 +772,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
                 prm_n0 = n0;
             }
             const int groups = (k_blocks + TC_GROUP - 1) / TC_GROUP;
-            if (!CELL && groups == 1 && prm.tma_epi != 0) {
+            if (!CELL && !PARTS && groups == 1 && prm.tma_epi != 0) {
                 // ---- one accumulator group: the blocks read tensor memory themselves (epi_block_direct) ----
                 if (!mbar_wait(tfull_bar(acc), acc_phase, abort_flag, 4)) { ok = false; break; }
                 tc_fence_after();
@@ -722,7 +788,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
                 if (res_ahead) {
                     res_ready = false;
                     const uint32_t next = tile + gridDim.x;
-                    if (next < tiles) {
+                    if (next < units) {
                         const TileGeom gn = geom_of(next);
                         if (gn.tma_tile && gn.box_in) {
                             if (lane == 0) {
@@ -846,7 +912,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
                 // request the next tile's residual blocks into the other half of the ring
                 res_ready = false;
                 const uint32_t next = tile + gridDim.x;
-                if (next < tiles) {
+                if (next < units) {
                     const TileGeom gn = geom_of(next);
                     if (gn.tma_tile && gn.box_in) {
                         if (lane == 0) {
@@ -1031,7 +1097,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
             __syncwarp();
             pending = -1;
         };
-        for (uint32_t tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
+        for (uint32_t unit = blockIdx.x; unit < units && ok; unit += gridDim.x) {
+            const int k_blocks = unit_blocks(unit);
             for (int kb = 0; kb < k_blocks; ++kb, ++kg) {
                 if ((int)(kg & (uint32_t)(TC_TEAMS - 1)) == team) {
                     // the raw tile has landed
@@ -1150,6 +1217,24 @@ CUtensorMap make_map_out(const float* base, int64_t B, int Ho, int Wo, int N, in
     return m;
 }
 
+// 5-D map over the group sums [groups][B][Ho][Wo][N] of a product, box as in make_map_out.
+CUtensorMap make_map_parts(const float* base, int64_t groups, int64_t B, int Ho, int Wo, int N, int wb, int hb) {
+    EncodeFn enc = tc_get_encode();
+    ensure(enc != nullptr, "cuTensorMapEncodeTiled is not available from this driver");
+    const int qw = std::min(wb, 32), qh = std::min(hb, 32 / qw), qn = 32 / (qw * qh);
+    CUtensorMap m;
+    const cuuint64_t row = (cuuint64_t)N * sizeof(float);
+    const cuuint64_t dims[5] = {(cuuint64_t)N, (cuuint64_t)Wo, (cuuint64_t)Ho, (cuuint64_t)B, (cuuint64_t)groups};
+    const cuuint64_t strides[4] = {row, row * (cuuint64_t)Wo, row * (cuuint64_t)Wo * (cuuint64_t)Ho, row * (cuuint64_t)Wo * (cuuint64_t)Ho * (cuuint64_t)B};
+    const cuuint32_t box[5] = {(cuuint32_t)TC_BK, (cuuint32_t)qw, (cuuint32_t)qh, (cuuint32_t)qn, 1u};
+    const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+    const CUresult r = enc(&m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 5, const_cast<float*>(base), dims, strides, box, estr,
+                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    ensure(r == CUDA_SUCCESS, "cuTensorMapEncodeTiled (group sums) failed with code " + std::to_string((int)r));
+    return m;
+}
+
 // Pixel box of an output tile: powers of two (Wb, Hb, Nb) with product 128 that need the fewest tiles.
 void choose_box(const ConvTcGeom& g, int& wb_log, int& hb_log, int& nb_log, int max_nb_log = 7) {
     int64_t best = -1;
@@ -1174,10 +1259,16 @@ struct CellState {
     int U = 0;
 };
 
-template <int BN, bool CELL = false>
+struct PartsOut {
+    float* base = nullptr;
+    int runs = 1, kb_run = 0;
+};
+
+template <int BN, int MODE = TC_PRODUCT>
 void launch_tc(const float* in, const ConvTcGeom& g, const float* Wb, const float* Ws, int64_t ldw, float* C, int64_t ldc, int N,
-               const Epilogue& e, cudaStream_t s, const CellState* cell = nullptr) {
+               const Epilogue& e, cudaStream_t s, const CellState* cell = nullptr, const PartsOut* parts = nullptr) {
     using Cfg = TcCfg<BN>;
+    constexpr bool CELL = MODE == TC_CELL, PARTS = MODE == TC_PARTS;
     {
         // the attribute belongs to the function on one device: set it once per device
         static std::mutex mu;
@@ -1186,7 +1277,7 @@ void launch_tc(const float* in, const ConvTcGeom& g, const float* Wb, const floa
         FDK_CUDA(cudaGetDevice(&dev));
         std::lock_guard<std::mutex> lock(mu);
         if (dev < 0 || dev >= 64 || !attr_set[dev]) {
-            FDK_CUDA(cudaFuncSetAttribute(gemm_tc_kernel<BN, CELL>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::MAX_SMEM));
+            FDK_CUDA(cudaFuncSetAttribute(gemm_tc_kernel<BN, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::MAX_SMEM));
             if (dev >= 0 && dev < 64) attr_set[dev] = true;
         }
     }
@@ -1230,14 +1321,20 @@ void launch_tc(const float* in, const ConvTcGeom& g, const float* Wb, const floa
                    ((prm.out_sx | prm.out_sy | prm.out_sb) & 3) == 0 &&
                    (e.residual == nullptr || ((e.ldr & 3) == 0 && (reinterpret_cast<uintptr_t>(e.residual) & 15) == 0))) ? 1 : 0;
     CUtensorMap mC = mA, mR = mA;  // placeholders when the TMA epilogue is off (never dereferenced then)
-    if (prm.tma_epi) {
+    prm.runs = 1; prm.kb_run = prm.taps * prm.cchunks;
+    if (PARTS) {
+        ensure(parts != nullptr && !volume && !spread && (N & 3) == 0, "internal: group sums need a dense 2-D product");
+        prm.runs = parts->runs; prm.kb_run = parts->kb_run;
+        prm.tma_epi = 1;
+        mC = make_map_parts(parts->base, (prm.taps * prm.cchunks + TC_GROUP - 1) / TC_GROUP, out_slices, g.Ho, g.Wo, N, 1 << wb, 1 << hb);
+    } else if (prm.tma_epi) {
         mC = make_map_out(C, out_slices, g.Ho, g.Wo, N, prm.out_sx, prm.out_sy, prm.out_sb, 1 << wb, 1 << hb);
         if (e.residual) {
             if (spread) mR = make_map_out(e.residual, out_slices, g.Ho, g.Wo, N, prm.out_sx, prm.out_sy, prm.out_sb, 1 << wb, 1 << hb);
             else mR = make_map_out(e.residual, out_slices, g.Ho, g.Wo, N, e.ldr, (int64_t)g.Wo * e.ldr, (int64_t)g.Ho * g.Wo * e.ldr, 1 << wb, 1 << hb);
         }
     }
-    const int64_t tiles = (int64_t)prm.tiles_w * prm.tiles_h * prm.tiles_n * ((N + BN - 1) / BN);
+    const int64_t tiles = (int64_t)prm.tiles_w * prm.tiles_h * prm.tiles_n * ((N + BN - 1) / BN) * prm.runs;  // work units
     ensure(tiles < (int64_t)1 << 31, "tensor-core kernel: too many tiles");
     const int grid = (int)std::min<int64_t>(tiles, tc_sm_count());
     // Shared memory plan (227 KB): staging buffers per epilogue warp (ring of 4 KB blocks), W stages and the raw A
@@ -1248,14 +1345,14 @@ void launch_tc(const float* in, const ConvTcGeom& g, const float* Wb, const floa
     const int k_blocks = prm.taps * prm.cchunks;
     const int n_tiles = (N + BN - 1) / BN;
     constexpr int NSUB = BN / 64;
-    const bool thin = k_blocks <= 4;
+    const bool thin = k_blocks <= 4 || PARTS;   // PARTS: a block of output per group
     if (!prm.tma_epi) prm.nbuf = 1;
     else if (e.residual) prm.nbuf = (thin || NSUB == 1) ? 2 * NSUB : NSUB;
     else prm.nbuf = thin ? (BN == 64 ? 4 : 2) : (BN == 64 ? 2 : 1);
     prm.stages = Cfg::STAGES;
     prm.a_stages = Cfg::A_STAGES;
     const int k_even = (k_blocks + 1) & ~1;
-    prm.w_stationary = (k_even <= Cfg::STAGES && (tiles <= grid || grid % n_tiles == 0)) ? 1 : 0;
+    prm.w_stationary = (!PARTS && k_even <= Cfg::STAGES && (tiles <= grid || grid % n_tiles == 0)) ? 1 : 0;
     prm.w_stages = prm.w_stationary ? k_even : prm.stages;
     // Shrink until it fits, keeping both rings at three stages or more as long as possible (a ring of two leaves
     // the ~1 us of a TMA load exposed at every other k block): A to 3, W to 3, then A to 2, W to 2, then the staging.
@@ -1278,7 +1375,7 @@ void launch_tc(const float* in, const ConvTcGeom& g, const float* Wb, const floa
     ensure(smem_bytes <= Cfg::MAX_SMEM, "tensor-core kernel: shared memory budget exceeded");
     if (CELL) ensure(cell != nullptr && prm.tma_epi != 0 && e.residual != nullptr && N % 64 == 0 && g.Ho == 1 && g.Wo == 1 && nb == 7,
                      "internal: the LSTM step kernel needs the TMA epilogue form");
-    launch_pdl(gemm_tc_kernel<BN, CELL>, dim3((unsigned)grid), dim3(TC_THREADS), (size_t)smem_bytes, s, mA, mWb, mWs, mC, mR, prm);
+    launch_pdl(gemm_tc_kernel<BN, MODE>, dim3((unsigned)grid), dim3(TC_THREADS), (size_t)smem_bytes, s, mA, mWb, mWs, mC, mR, prm);
 }
 
 }  // namespace
@@ -1321,6 +1418,177 @@ static ConvTcGeom gemm_geom(int64_t M, int K, int64_t lda) {
     return g;
 }
 
+// ---- products of few rows: group sums first, then their sum ------------------------------------------------
+// A tile walks its k blocks one after the other at about 1000 cycles each whatever the rest of the chip does: one
+// ResNet-50 image has 4 to 98 tiles per layer for 148 SMs, and its 3 x 3 layers took 20 to 75 us each.  Spread over all SMs
+// the walk is 2 to 8 blocks long; the price is the group sums' trip through L2 (every group leaves separately, so that the
+// sum can be made in the order of the whole walk) and a second launch.  ResNet-50, one image from the host: 1230 -> 701 us;
+// three texts of 120 words through two LSTM layers: 3410 -> 2180 us; five MobileNetV2 images: 453 -> 410 us.
+namespace {
+
+int split_tiles(const ConvTcGeom& g, int N, int BN) {
+    int wb, hb, nb;
+    choose_box(g, wb, hb, nb);
+    const int64_t t = (int64_t)((g.Wo + (1 << wb) - 1) >> wb) * ((g.Ho + (1 << hb) - 1) >> hb) * ((g.B + (1 << nb) - 1) >> nb) * ((N + BN - 1) / BN);
+    return (int)std::min<int64_t>(t, 1 << 20);
+}
+
+// Adds the group sums of a product in group order, exactly as the epilogue warps of gemm_tc_kernel do when one CTA walks
+// the whole contraction, then applies the same epilogue: the results are the same bit for bit.
+// A block holds 256 / L float4 columns; L lanes per column fetch the groups together (shared memory), because a chain of
+// dependent loads, not bandwidth, is what a few thousand values with up to 72 groups each would wait for.
+template <int L>
+__global__ void __launch_bounds__(256) sum_parts_kernel(const float* __restrict__ parts, long long pitch, int groups, float* __restrict__ C,
+                                                        long long ldc, int n4, long long total4, EpiDev e, int aligned) {
+    constexpr int COLS = 256 / L;
+    extern __shared__ float4 sp_sum[];
+    pdl_launch_dependents();
+    pdl_wait();
+    const float4* p = reinterpret_cast<const float4*>(parts);
+    const long long pitch4 = pitch >> 2;
+    for (long long c0 = (long long)blockIdx.x * COLS; c0 < total4; c0 += (long long)gridDim.x * COLS) {
+        const int col = threadIdx.x % COLS, l = threadIdx.x / COLS;
+        const long long i = c0 + col;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (L == 1) {
+            if (i < total4) {
+                v = __ldcg(p + i);
+#pragma unroll 8
+                for (int g = 1; g < groups; ++g) {
+                    const float4 t = __ldcg(p + (long long)g * pitch4 + i);
+                    v.x += t.x; v.y += t.y; v.z += t.z; v.w += t.w;
+                }
+            }
+        } else {
+            if (i < total4) {
+#pragma unroll 8
+                for (int g = l; g < groups; g += L) sp_sum[g * COLS + col] = __ldcg(p + (long long)g * pitch4 + i);
+            }
+            __syncthreads();
+            if (l == 0 && i < total4) {
+                v = sp_sum[col];
+#pragma unroll 8
+                for (int g = 1; g < groups; ++g) {
+                    const float4 t = sp_sum[g * COLS + col];
+                    v.x += t.x; v.y += t.y; v.z += t.z; v.w += t.w;
+                }
+            }
+            __syncthreads();
+        }
+        if (l == 0 && i < total4) {
+            const long long row = i / n4;
+            const int n = (int)(i - row * n4) * 4;
+            float o[4] = {v.x, v.y, v.z, v.w};
+            if (aligned) {
+                // the form of the epilogue through TMA: absent parameters are 0, 1, 0
+                const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
+                const float4 b = e.bias ? __ldg(reinterpret_cast<const float4*>(e.bias + n)) : z4;
+                const float4 sc = e.scale ? __ldg(reinterpret_cast<const float4*>(e.scale + n)) : make_float4(1.f, 1.f, 1.f, 1.f);
+                const float4 sh = e.scale ? __ldg(reinterpret_cast<const float4*>(e.shift + n)) : z4;
+                const float bb[4] = {b.x, b.y, b.z, b.w}, ss[4] = {sc.x, sc.y, sc.z, sc.w}, tt[4] = {sh.x, sh.y, sh.z, sh.w};
+#pragma unroll
+                for (int k = 0; k < 4; ++k) o[k] = __fadd_rn(__fmul_rn(__fadd_rn(o[k], bb[k]), ss[k]), tt[k]);
+                if (e.residual) {
+                    const float4 r = __ldcg(reinterpret_cast<const float4*>(e.residual + row * e.ldr + n));
+                    o[0] += r.x; o[1] += r.y; o[2] += r.z; o[3] += r.w;
+                }
+                if (e.act2.kind != ACT_NONE) {
+                    const float hi = e.act2.kind == ACT_RELU_GEN ? e.act2.p0 : __int_as_float(0x7f800000);
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) o[k] = fminf(fmaxf(0.0f, o[k]), hi);
+                }
+                *reinterpret_cast<float4*>(C + row * ldc + n) = make_float4(o[0], o[1], o[2], o[3]);
+            } else {
+#pragma unroll 1
+                for (int k = 0; k < 4; ++k) C[row * ldc + n + k] = epi_apply(e, o[k], row, n + k);
+            }
+        }
+    }
+}
+
+// Model of the time, in microseconds: a k block of a tile takes 0.55 (one CTA, about 1000 cycles, whatever the tile's
+// width), a work unit 1.5 more; the group sums are written and read once at 4 TB/s, and adding them up is a launch.
+struct SplitPlan { int bn = 0, runs = 1, kb_run = 0; };
+SplitPlan split_plan(const ConvTcGeom& g, int N) {
+    SplitPlan best;
+    if (g.D > 1 || g.Do > 1 || g.kd > 1 || g.out_sx > 0 || (N & 3)) return best;
+    const bool rowwin = g.win_stride > 0;
+    const int k_blocks = rowwin ? g.kh : g.kh * g.kw * ((g.C + TC_BK - 1) / TC_BK);
+    if (k_blocks < 2 * TC_GROUP) return best;
+    const int sms = tc_sm_count();
+    const int tiles[2] = {split_tiles(g, N, 64), split_tiles(g, N, 128)};
+    if ((N <= 64 ? tiles[0] : tiles[1]) >= sms) return best;
+    const int64_t groups = (k_blocks + TC_GROUP - 1) / TC_GROUP, M = g.B * g.Ho * g.Wo;
+    if (groups > 128 || groups * M * N > SPLIT_MAX_FLOATS) return best;   // 128: sum_parts_kernel's shared memory
+    const int whole_tiles = (N <= 64 || tiles[1] * 2 <= sms) ? tiles[0] : tiles[1];
+    auto waves = [&](int64_t units) { return (double)((units + sms - 1) / sms); };
+    double least = 0.85 * waves(whole_tiles) * (1.5 + 0.55 * k_blocks);   // a split has to be worth its second launch
+    const double sums = 2.5 + 8.0 * (double)groups * (double)M * N / 4e6;
+    for (int w = 0; w < (N <= 64 ? 1 : 2); ++w)
+        for (int run = TC_GROUP; run * 2 <= k_blocks + TC_GROUP - 1; run += TC_GROUP) {
+            const int runs = (k_blocks + run - 1) / run;
+            const double t = waves((int64_t)tiles[w] * runs) * (1.5 + 0.55 * run) + sums;
+            if (t < least) { least = t; best.bn = w ? 128 : 64; best.runs = runs; best.kb_run = run; }
+        }
+    return best;
+}
+
+void launch_parts(const float* in, const ConvTcGeom& g, const float* Wbig, const float* Wsmall, int64_t ldw, int N, const SplitPlan& plan, float* parts,
+                  cudaStream_t s) {
+    PartsOut out{parts, plan.runs, plan.kb_run};
+    const Epilogue none;
+    if (plan.bn == 64) launch_tc<64, TC_PARTS>(in, g, Wbig, Wsmall, ldw, parts, N, N, none, s, nullptr, &out);
+    else launch_tc<128, TC_PARTS>(in, g, Wbig, Wsmall, ldw, parts, N, N, none, s, nullptr, &out);
+}
+
+}  // namespace
+
+int64_t conv_tc_parts_floats(const ConvTcGeom& g, int N) {
+    const SplitPlan plan = split_plan(g, N);
+    if (plan.runs < 2) return 0;
+    const int k_blocks = g.win_stride > 0 ? g.kh : g.kh * g.kw * ((g.C + TC_BK - 1) / TC_BK);
+    return (int64_t)((k_blocks + TC_GROUP - 1) / TC_GROUP) * g.B * g.Ho * g.Wo * N;
+}
+int64_t gemm_tc_parts_floats(int64_t M, int N, int K) { return conv_tc_parts_floats(gemm_geom(M, K, K), N); }
+
+void launch_conv_tc_parts(const float* in, const ConvTcGeom& g, const float* Wbig, const float* Wsmall, int64_t ldw, float* C, int64_t ldc, int N,
+                          const Epilogue& epilogue, float* parts, cudaStream_t s) {
+    const SplitPlan plan = split_plan(g, N);
+    ensure(plan.runs > 1 && parts != nullptr, "internal: this product is not split");
+    launch_parts(in, g, Wbig, Wsmall, ldw, N, plan, parts, s);
+    Epilogue e = epilogue;
+    if (e.scale == nullptr && e.residual == nullptr && e.act2.none()) std::swap(e.act1, e.act2);
+    const bool plain_act = e.act1.kind == ACT_NONE &&
+                           (e.act2.kind == ACT_NONE || e.act2.kind == ACT_RELU || (e.act2.kind == ACT_RELU_GEN && e.act2.p1 == 0.0f && e.act2.p2 == 0.0f));
+    auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
+    const int aligned = plain_act && (ldc & 3) == 0 && al16(C) && (e.residual == nullptr || ((e.ldr & 3) == 0 && al16(e.residual))) && al16(e.bias) &&
+                        al16(e.scale) && al16(e.shift);
+    const int64_t M = g.B * g.Ho * g.Wo, total4 = M * N / 4;
+    const int groups = (int)((g.win_stride > 0 ? g.kh : g.kh * g.kw * ((g.C + TC_BK - 1) / TC_BK)) + TC_GROUP - 1) / TC_GROUP;
+    // lanes per column: enough loads in flight for few values or many groups
+    const int lanes = total4 >= 148 * 256 && groups <= 16 ? 1 : groups <= 16 ? 4 : 16;
+    const int cols = 256 / lanes;
+    const unsigned grid = (unsigned)std::min<int64_t>((total4 + cols - 1) / cols, 148 * 16);
+    const size_t smem = lanes == 1 ? 0 : (size_t)groups * cols * sizeof(float4);
+    ensure(smem <= 48 * 1024, "internal: too many group sums for one block");
+    auto kernel = lanes == 1 ? sum_parts_kernel<1> : lanes == 4 ? sum_parts_kernel<4> : sum_parts_kernel<16>;
+    launch_pdl(kernel, dim3(grid), dim3(256), smem, s, (const float*)parts, (long long)(M * N), groups, C, (long long)ldc, N / 4, (long long)total4,
+               to_dev(e), aligned);
+}
+
+void launch_gemm_tc_parts(const float* A, int64_t lda, const float* Wbig, const float* Wsmall, int64_t ldw, float* C, int64_t ldc, int64_t M, int N,
+                          int K, const Epilogue& e, float* parts, cudaStream_t s) {
+    launch_conv_tc_parts(A, gemm_geom(M, K, lda), Wbig, Wsmall, ldw, C, ldc, N, e, parts, s);
+}
+int launch_gemm_tc_group_sums(const float* A, int64_t lda, const float* Wbig, const float* Wsmall, int64_t ldw, int64_t M, int N, int K, float* parts,
+                              cudaStream_t s) {
+    const ConvTcGeom g = gemm_geom(M, K, lda);
+    const SplitPlan plan = split_plan(g, N);
+    ensure(plan.runs > 1 && parts != nullptr, "internal: this product is not split");
+    launch_parts(A, g, Wbig, Wsmall, ldw, N, plan, parts, s);
+    return ((K + TC_BK - 1) / TC_BK + TC_GROUP - 1) / TC_GROUP;
+}
+
 bool gemm_tc_supported(int64_t M, int N, int K, int64_t lda, int64_t ldw, const void* A, const void* W) {
     if (M <= 0 || K <= 0) return false;
     return conv_tc_supported(gemm_geom(M, K, lda), N, ldw, A, W);
@@ -1346,7 +1614,7 @@ void launch_lstm_step_tc(const float* h, const float* Wbig, const float* Wsmall,
     e.ldr = ldx;
     CellState cell;
     cell.c = c; cell.h = h_next; cell.out = out; cell.out_stride = out_stride; cell.U = U;
-    launch_tc<128, true>(h, gemm_geom(B, U, U), Wbig, Wsmall, ldw, z_unused, (int64_t)4 * U, 4 * U, e, s, &cell);
+    launch_tc<128, TC_CELL>(h, gemm_geom(B, U, U), Wbig, Wsmall, ldw, z_unused, (int64_t)4 * U, 4 * U, e, s, &cell);
 }
 
 const int* gemm_tc_status_address() {

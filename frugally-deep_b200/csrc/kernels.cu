@@ -1435,6 +1435,39 @@ __global__ void __launch_bounds__(256) lstm_cellv_kernel(const float* __restrict
         if (out) *reinterpret_cast<Vec*>(out + (int64_t)b * out_stride + V * j) = hn;
     }
 }
+// The same step where the recurrent product left its group sums: they are added in group order, the input's row last, as
+// the product's epilogue does, so the results are those of the form with the product finished.  One unit per thread, the
+// loads of its four gates in flight together.
+__global__ void __launch_bounds__(64) lstm_cell_parts_kernel(const float* __restrict__ parts, int groups, const float* __restrict__ x, int64_t ldx,
+                                                             float* __restrict__ c, float* __restrict__ h, float* __restrict__ out, int64_t out_stride,
+                                                             int total, int U) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int64_t pitch = (int64_t)total * 4;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+        const int b = i / U;
+        const int j = i - b * U;
+        const float* p = parts + (int64_t)b * 4 * U + j;
+        float z[4], xv[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) xv[k] = __ldcg(x + b * ldx + k * U + j);
+        const float cv = __ldcg(c + i);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) z[k] = __ldcg(p + k * U);
+#pragma unroll 8
+        for (int g = 1; g < groups; ++g) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) z[k] += __ldcg(p + g * pitch + k * U);
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) z[k] = __fadd_rn(__fadd_rn(z[k], 0.0f), xv[k]);
+        const float cn = __fadd_rn(__fmul_rn(sigmoid_ref(z[1]), cv), __fmul_rn(sigmoid_ref(z[0]), tanhf(z[2])));
+        const float hn = __fmul_rn(sigmoid_ref(z[3]), tanhf(cn));
+        c[i] = cn;
+        h[i] = hn;
+        if (out) out[b * out_stride + j] = hn;
+    }
+}
 __global__ void gru_cell_kernel(const float* __restrict__ xw, int64_t ldx, const float* __restrict__ hu, float* __restrict__ h,
                                 float* __restrict__ out, int64_t out_stride, int64_t total, int U, ActSpecDev act, ActSpecDev ract) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
@@ -1495,6 +1528,13 @@ void launch_gru_out(const float* xw, int64_t ldx, const float* zr, int64_t ldh, 
     FDK_CUDA(cudaGetLastError());
 }
 
+bool launch_lstm_cell_parts(const float* parts, int groups, const float* x, int64_t ldx, float* c, float* h, float* out, int64_t out_stride, int64_t B,
+                            int U, ActSpec act, ActSpec ract, cudaStream_t s) {
+    const int64_t total = B * U;
+    if (act.kind != ACT_TANH || ract.kind != ACT_SIGMOID || total <= 0 || total > 0x1fffffffLL) return false;
+    launch_pdl(lstm_cell_parts_kernel, dim3((unsigned)((total + 63) / 64)), dim3(64), 0, s, parts, groups, x, ldx, c, h, out, out_stride, (int)total, U);
+    return true;
+}
 void launch_lstm_cell(const float* z, float* c, float* h, float* out, int64_t out_stride, int64_t B, int U, ActSpec act,
                       ActSpec ract, cudaStream_t s) {
     const int64_t total = B * U;

@@ -81,6 +81,19 @@ struct ConvTcGeom {
 bool conv_tc_supported(const ConvTcGeom& g, int N, int64_t ldw, const void* in, const void* W);
 void launch_conv_tc(const float* in, const ConvTcGeom& g, const float* Wbig, const float* Wsmall, int64_t ldw, float* C,
                     int64_t ldc, int N, const Epilogue& e, cudaStream_t s);
+// The same product for few rows, whose tiles would leave most SMs idle while each walks its contraction alone: the k blocks
+// of a tile are spread over CTAs, which leave the sums of their accumulator groups in `parts`, and a second kernel adds
+// them in the order in which one CTA would have: the results do not change by a bit, so the choice may depend on the
+// batch.  *_parts_floats: floats of `parts` such a launch needs, 0 where the whole product is the better form.
+int64_t conv_tc_parts_floats(const ConvTcGeom& g, int N);
+int64_t gemm_tc_parts_floats(int64_t M, int N, int K);
+void launch_conv_tc_parts(const float* in, const ConvTcGeom& g, const float* Wbig, const float* Wsmall, int64_t ldw, float* C, int64_t ldc, int N,
+                          const Epilogue& e, float* parts, cudaStream_t s);
+void launch_gemm_tc_parts(const float* A, int64_t lda, const float* Wbig, const float* Wsmall, int64_t ldw, float* C, int64_t ldc, int64_t M, int N,
+                          int K, const Epilogue& e, float* parts, cudaStream_t s);
+// The first kernel alone; returns the number of group sums, [groups][M][N] in `parts`.
+int launch_gemm_tc_group_sums(const float* A, int64_t lda, const float* Wbig, const float* Wsmall, int64_t ldw, int64_t M, int N, int K, float* parts,
+                              cudaStream_t s);
 // One LSTM time step in one launch: z = h U + x (x = this step's rows of the input product, bias included) never
 // leaves the SM; the epilogue applies the cell (tanh / sigmoid) and writes c in place, the new h to h_next (a buffer
 // other than h: other CTAs still read h) and, if given, to out.  U's rows (and x's columns) must be in the cell order:
@@ -174,6 +187,10 @@ void launch_embedding(const float* ids, const float* table, float* out, int64_t 
                       int* err, cudaStream_t s);
 // ---- recurrent cells -----------------------------------------------------------------------------------
 // z[B,4U] holds x_t W + b + h U (gate order i, f, c~, o); updates c and h in place, writes h to out rows.
+// Cell step on the group sums [groups][B][4U] of the recurrent product (launch_gemm_tc_group_sums) and this step's input
+// rows x (row stride ldx).  Standard activations only: returns false (nothing launched) for others.
+bool launch_lstm_cell_parts(const float* parts, int groups, const float* x, int64_t ldx, float* c, float* h, float* out, int64_t out_stride, int64_t B,
+                            int U, ActSpec act, ActSpec ract, cudaStream_t s);
 void launch_lstm_cell(const float* z, float* c, float* h, float* out, int64_t out_stride, int64_t B, int U,
                       ActSpec act, ActSpec ract, cudaStream_t s);
 // GRU with reset_after: xw[B,3U] (= x W + b_x, row stride ldx), hu[B,3U] (= h U + b_h); order z, r, h~.

@@ -1036,3 +1036,78 @@ def test_category_encoding_value_outside_raises(built_library):
     with pytest.raises(fdeep_b200.FdeepError, match="num_tokens"):
         m.predict([np.array([0.0, 4.0, 1.0], np.float32)])
     m.predict([np.array([2.0, 3.0, 1.0], np.float32)])  # the context stays usable
+
+
+# (input side, channels, filters, kernel, stride): k blocks 10 (ragged last), 18 with a partial channel chunk, 72, 16, 50;
+# columns that are no multiple of 32 or 64; one row of the tile, one partial tile, several tiles
+SPLIT_SHAPES = [(1, 300, 68, 1, 1), (7, 40, 256, 3, 1), (7, 256, 512, 3, 1), (14, 512, 36, 1, 1), (15, 64, 100, 5, 2)]
+
+
+@pytest.mark.parametrize("side,cin,cout,k,stride", SPLIT_SHAPES)
+@pytest.mark.parametrize("tail", ["none", "bn_add_relu", "sigmoid"])
+def test_few_rows_spread_over_the_k_blocks(built_library, side, cin, cout, k, stride, tail):
+    """A convolution on few rows spreads the k blocks of a tile over CTAs and adds the group sums in a second launch
+    (fdk::launch_conv_tc_parts); a large batch walks each tile whole.  Same sample, same bits, whatever follows the product
+    (nothing, BatchNormalization + residual + ReLU, an activation that takes the epilogue for odd rows), and both against the
+    oracle."""
+    rng = np.random.default_rng(side * 1000 + cin + cout)
+    b = mw.ModelBuilder("m")
+    i = b.input([side, side, cin])
+    kernel = rng.normal(size=(k, k, cin, cout)).astype(np.float32) / np.sqrt(k * k * cin)
+    y = mw.conv2d(b, i, "c", kernel, rng.normal(size=cout).astype(np.float32), strides=stride, padding="same",
+                  activation="sigmoid" if tail == "sigmoid" else "linear")
+    out_side = -(-side // stride)
+    inputs, in_shapes = [i], [[side, side, cin]]
+    if tail == "bn_add_relu":
+        j = b.input([out_side, out_side, cout])
+        in_shapes.append([out_side, out_side, cout])
+        y = mw.batch_norm(b, y, "bn", rng.normal(size=cout).astype(np.float32), rng.uniform(0.5, 2, cout).astype(np.float32),
+                          rng.uniform(0.5, 2, cout).astype(np.float32), rng.normal(size=cout).astype(np.float32))
+        y = mw.relu(b, mw.add_layers(b, [y, j], "add"), "relu")
+    text = model_text(b.to_json([y], [[out_side, out_side, cout]]))
+    many = 148 * 128 // (out_side * out_side) + 1
+    pool = [[rng.normal(size=s).astype(np.float32) for s in in_shapes] for _ in range(4)]
+    m = fdeep_b200.read_model_from_string(text, verify=False)
+    few = [o[0] for o in m.predict_multi(pool[:1])]
+    large = m.predict_multi([pool[s % 4] for s in range(many)])
+    want = oracle_outputs(text, pool[:1])
+    np.testing.assert_array_equal(few[0], large[0][0])
+    np.testing.assert_array_equal(few[0], large[many - many % 4 - 4][0])
+    assert_close(few[0], want[0][0], f"{side}x{side}x{cin} -> {cout}, {k}x{k}/{stride}, {tail}")
+    twice = m.predict_multi(pool[:1])   # (the group sums of the call before are still in the workspace)
+    np.testing.assert_array_equal(few[0], twice[0][0])
+    import torch
+    launches = []
+    for n in (1, many):
+        x = [torch.zeros([n] + s, device="cuda") for s in in_shapes]
+        out = torch.empty([n, out_side, out_side, cout], device="cuda")
+        torch.cuda.synchronize()
+        before = m.launch_count()
+        m.predict_batch_device([t.data_ptr() for t in x], in_shapes, n, [out.data_ptr()])
+        m.sync()
+        launches.append(m.launch_count() - before)
+    assert launches[0] == launches[1] + 1, f"few rows: {launches[0]} launches, many: {launches[1]}"
+
+
+@pytest.mark.parametrize("units,samples", [(256, 1), (512, 3), (500, 37), (512, 300)])
+def test_lstm_step_on_group_sums(built_library, units, samples):
+    """LSTM steps on few rows: the cell kernel adds the recurrent product's group sums itself; 300 samples run as two chains
+    with a part of the workspace each.  Against the same sequences in a batch whose tiles fill the device, bit for bit."""
+    rng = np.random.default_rng(units + samples)
+    T, F = 5, 12
+    b = mw.ModelBuilder("m")
+    i = b.input([T, F])
+    W = rng.normal(size=(F, 4 * units)).astype(np.float32) * 0.4
+    U = rng.normal(size=(units, 4 * units)).astype(np.float32) * (1.5 / np.sqrt(units))
+    text = model_text(b.to_json([mw.lstm(b, i, "l", W, U, rng.normal(size=4 * units).astype(np.float32) * 0.1, return_sequences=True)], [[T, units]]))
+    xs = [[rng.normal(size=(T, F)).astype(np.float32)] for _ in range(samples)]
+    m = fdeep_b200.read_model_from_string(text, verify=False)
+    few = m.predict_multi(xs)
+    again = m.predict_multi(xs)
+    many = m.predict_multi([xs[s % samples] for s in range(2700)])
+    want = oracle_outputs(text, xs[:3])
+    for s in range(samples):
+        np.testing.assert_array_equal(few[s][0], many[s][0])
+        np.testing.assert_array_equal(few[s][0], again[s][0])
+        if s < 3:
+            assert_close(few[s][0], want[s][0], f"{units} units, sample {s}")

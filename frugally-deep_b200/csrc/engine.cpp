@@ -84,6 +84,7 @@ Engine::~Engine() {
         cudaFree(c->w.base);
         cudaFree(c->arena);
         cudaFree(c->in_stage);
+        cudaFree(c->device_stage);
         cudaFree(c->byte_stage);
         cudaFree(c->workspace);
         cudaFree(c->d_err);
@@ -1220,20 +1221,57 @@ void Engine::predict_batch_device(int dev_index, int64_t batch, const float* con
             FDK_CUDA(cudaMemcpyAsync(d_out[o], src, sizeof(float) * (size_t)(batch * t.shape.volume()), cudaMemcpyDeviceToDevice, on));
         }
     };
-    if (!live || profile || kv) {
+    // A small call is replayed on memory of the engine, one copy in and one out per tensor: what is recorded knows nothing of
+    // the caller's buffers, so new ones cost no more than the last call's.  Above DEVICE_STAGE_FLOATS (4 MB: a copy of about
+    // 3 us, 60 launches cost 200 us of host time) the device is busy for longer than the launches take to queue.
+    bool staged = live && !profile && !kv;
+    int64_t floats = 0;
+    auto reserve = [&](const void* q, int64_t n) {
+        const int64_t at = floats;
+        floats += round_up64(n, 64);
+        staged = staged && (reinterpret_cast<uintptr_t>(q) & 15) == 0 && floats <= DEVICE_STAGE_FLOATS;   // odd addresses: as they always were
+        return at;
+    };
+    std::vector<int64_t> in_at, out_at;
+    for (size_t i = 0; i < p->inputs.size(); ++i) in_at.push_back(reserve(d_in[i], batch * p->in_shapes[i].volume()));
+    for (size_t o = 0; o < p->outputs.size(); ++o)
+        out_at.push_back(d_out[o] ? reserve(d_out[o], batch * p->tensors[(size_t)p->outputs[o]].shape.volume()) : 0);
+    if (staged && !c.device_stage && cudaMalloc(&c.device_stage, sizeof(float) * DEVICE_STAGE_FLOATS) != cudaSuccess) {
+        cudaGetLastError();
+        c.device_stage = nullptr;
+    }
+    if (!staged || !c.device_stage) {
         queue(s);
     } else {
-        std::vector<const void*> where(d_in, d_in + p->inputs.size());
-        where.insert(where.end(), d_out, d_out + p->outputs.size());
+        std::vector<const float*> st_in;
+        std::vector<float*> st_out;
+        for (size_t i = 0; i < p->inputs.size(); ++i) {
+            st_in.push_back(c.device_stage + in_at[i]);
+            FDK_CUDA(cudaMemcpyAsync(c.device_stage + in_at[i], d_in[i], sizeof(float) * (size_t)(batch * p->in_shapes[i].volume()), cudaMemcpyDefault, s));
+        }
+        for (size_t o = 0; o < p->outputs.size(); ++o) st_out.push_back(d_out[o] ? c.device_stage + out_at[o] : nullptr);
+        std::vector<const void*> where(st_in.begin(), st_in.end());
+        where.insert(where.end(), st_out.begin(), st_out.end());
+        const float* const* caller_in = d_in;
+        float* const* caller_out = d_out;
+        d_in = st_in.data();
+        d_out = st_out.data();
         replay(c, *p, batch, std::move(where), 0.f, 0.f, s, queue);
+        d_in = caller_in;
+        d_out = caller_out;
+        for (size_t o = 0; o < p->outputs.size(); ++o)
+            if (d_out[o])
+                FDK_CUDA(cudaMemcpyAsync(d_out[o], st_out[o], sizeof(float) * (size_t)(batch * p->tensors[(size_t)p->outputs[o]].shape.volume()),
+                                         cudaMemcpyDefault, s));
     }
     if (live) mark_use(c, s);
 }
 
-// A call repeated with the same plan, batch and addresses costs one graph launch instead of the launches of the plan (60 to
+// A call repeated with the same plan and batch (and the engine's buffers where they were) costs one graph launch instead of the launches of the plan (60 to
 // 800 of them, 3 to 6 us of host time each with their tensor maps, and gaps between short kernels).  The first call of a kind
 // runs directly (every buffer reaches its size), the second one is recorded.  At most 32 calls are kept per device; the
-// addresses of the arena and the workspace belong to the key because other calls may make them move.
+// addresses of the staging buffers, the arena and the workspace belong to the key because other calls may make them move.
+// No address of the caller's is ever part of a recording.
 template <typename F>
 void Engine::replay(DeviceCtx& c, const Plan& p, int64_t batch, std::vector<const void*> where, float low, float high, cudaStream_t s, F&& queue) {
     static const bool enabled = [] { const char* v = getenv("FDK_PREDICT_GRAPH"); return !(v && *v == '0'); }();

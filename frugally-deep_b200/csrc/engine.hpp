@@ -78,13 +78,15 @@ struct DeviceWeights {
 struct RecordedCall {
     const Plan* plan = nullptr;
     int64_t batch = 0;
-    std::vector<const void*> where;    // caller's buffers or staging buffers, arena, workspace
+    std::vector<const void*> where;    // staging buffers, arena, workspace
     float low = 0.f, high = 0.f;
     cudaGraphExec_t exec = nullptr;
     int64_t launches = 0;
     uint64_t last_use = 0;
     bool unusable = false;             // could not be recorded: launch directly
 };
+
+constexpr int64_t DEVICE_STAGE_FLOATS = 1 << 20;
 
 struct DeviceCtx {
     uint8_t* byte_stage = nullptr;   // device staging for byte inputs
@@ -100,6 +102,7 @@ struct DeviceCtx {
     int64_t arena_elems = 0;
     float* in_stage = nullptr;     // device staging for host inputs
     int64_t in_stage_elems = 0;
+    float* device_stage = nullptr; // inputs and outputs of small calls on device memory (DEVICE_STAGE_FLOATS), see predict_batch_device
     float* h_in = nullptr;         // pinned host staging
     int64_t h_in_elems = 0;
     float* h_out = nullptr;

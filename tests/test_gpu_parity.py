@@ -1111,3 +1111,22 @@ def test_lstm_step_on_group_sums(built_library, units, samples):
         np.testing.assert_array_equal(few[s][0], again[s][0])
         if s < 3:
             assert_close(few[s][0], want[s][0], f"{units} units, sample {s}")
+
+
+@pytest.mark.parametrize("n", [1, 37, 341, 342])
+def test_device_calls_on_ever_new_buffers(built_library, n):
+    """predict_batch_device replays small calls (up to 4 MB of inputs and outputs, 341 samples here) on memory of the engine:
+    every call with other buffers and other values gives what the host path gives, and what lies around the output stays."""
+    import torch
+    m, _ = load(mw.build_small_cnn(), True)
+    for rep in range(4):
+        x = np.random.default_rng(100 * n + rep).random((n, 32, 32, 3), dtype=np.float32)
+        d_in = torch.from_numpy(x).cuda()
+        d_out = torch.full((n + 2, 10), -7.0, device="cuda")
+        torch.cuda.synchronize()
+        m.predict_batch_device([d_in.data_ptr()], [[32, 32, 3]], n, [d_out[1:].data_ptr() if rep % 2 else d_out.data_ptr()])
+        m.sync()
+        got = d_out.cpu().numpy()
+        first = 1 if rep % 2 else 0   # (40 bytes on: not 16-byte aligned)
+        np.testing.assert_array_equal(got[first:first + n], m.predict_batch([x])[0])
+        assert (np.delete(got, np.s_[first:first + n], axis=0) == -7.0).all()

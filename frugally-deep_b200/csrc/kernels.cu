@@ -824,6 +824,41 @@ __global__ void global_pool_kernel(const float* __restrict__ in, float* __restri
         out[i] = is_max ? val : val / (float)spatial;
     }
 }
+// The same for more positions than a thread should walk on its own: a block fetches 32 channels x up to 128 positions with
+// all its threads (16 loads of a thread in flight), one warp adds them in the order of the walk, so the results are the
+// same.  The walk was a chain of dependent adds on loads of its own: 34 us for ONE sample of 16 x 16 x 64.
+constexpr int GP_POS = 128;
+__global__ void __launch_bounds__(256) global_pool_tiles_kernel(const float* __restrict__ in, float* __restrict__ out, int64_t blocks, int c_blocks,
+                                                                int64_t spatial, int C, bool is_max) {
+    __shared__ float tile[GP_POS][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (int64_t blk = blockIdx.x; blk < blocks; blk += gridDim.x) {
+        const int64_t b = blk / c_blocks;
+        const int c = (int)(blk - b * c_blocks) * 32 + lane;
+        const float* p = in + b * spatial * C + c;
+        float val = is_max ? -FLT_MAX : 0.f;
+        for (int64_t s0 = 0; s0 < spatial; s0 += GP_POS) {
+            const int n = (int)(spatial - s0 < GP_POS ? spatial - s0 : GP_POS);
+            if (c < C) {
+#pragma unroll
+                for (int k = 0; k < GP_POS / 8; ++k)
+                    if (w + 8 * k < n) tile[w + 8 * k][lane] = p[(s0 + w + 8 * k) * C];
+            }
+            __syncthreads();
+            if (w == 0 && c < C) {
+                if (is_max) {
+#pragma unroll 16
+                    for (int k = 0; k < n; ++k) val = fmaxf(val, tile[k][lane]);
+                } else {
+#pragma unroll 16
+                    for (int k = 0; k < n; ++k) val += tile[k][lane];
+                }
+            }
+            __syncthreads();
+        }
+        if (w == 0 && c < C) out[b * C + c] = is_max ? val : val / (float)spatial;
+    }
+}
 }  // namespace
 
 void launch_pool3d(const float* in, float* out, int64_t B, int D, int H, int W, int C, int Do, int Ho, int Wo, int pd, int ph,
@@ -850,7 +885,11 @@ void launch_pool3d(const float* in, float* out, int64_t B, int D, int H, int W, 
 }
 void launch_global_pool(const float* in, float* out, int64_t B, int64_t spatial, int C, bool is_max, cudaStream_t s) {
     if (B * C == 0) return;
-    global_pool_kernel<<<grid_1d(B * C, 128), 128, 0, s>>>(in, out, B, spatial, C, is_max);
+    const int c_blocks = (C + 31) / 32;
+    const int64_t blocks = B * c_blocks;
+    // a handful of positions, or mostly idle lanes: a thread per channel walks them
+    if (spatial <= 8 || C < 16) global_pool_kernel<<<grid_1d(B * C, 128), 128, 0, s>>>(in, out, B, spatial, C, is_max);
+    else global_pool_tiles_kernel<<<(unsigned)std::min<int64_t>(blocks, 148 * 64), 256, 0, s>>>(in, out, blocks, c_blocks, spatial, C, is_max);
     FDK_CUDA(cudaGetLastError());
 }
 

@@ -1130,3 +1130,18 @@ def test_device_calls_on_ever_new_buffers(built_library, n):
         first = 1 if rep % 2 else 0   # (40 bytes on: not 16-byte aligned)
         np.testing.assert_array_equal(got[first:first + n], m.predict_batch([x])[0])
         assert (np.delete(got, np.s_[first:first + n], axis=0) == -7.0).all()
+
+
+@pytest.mark.parametrize("side,channels", [((3, 3), 16), ((8, 16), 33), ((3, 43), 64), ((17, 23), 1280)])
+@pytest.mark.parametrize("kind", ["GlobalAveragePooling2D", "GlobalMaxPooling2D"])
+def test_global_pooling_tiles(built_library, side, channels, kind):
+    """Global pooling by blocks of 32 channels x 128 positions (9, 128, 129 and 391 positions; channels that fill no block):
+    the positions are added in order in 32 bits, so numpy's running sum has the same bits."""
+    b = mw.ModelBuilder("m")
+    i = b.input([*side, channels])
+    y = b.add(kind, "p", {"data_format": "channels_last", "keepdims": False}, [i])
+    m = fdeep_b200.read_model_from_string(model_text(b.to_json([y], [[channels]])), verify=False)
+    x = np.random.default_rng(channels).normal(size=(5, *side, channels)).astype(np.float32)
+    rows = x.reshape(5, -1, channels)
+    want = rows.max(axis=1) if "Max" in kind else np.cumsum(rows, axis=1, dtype=np.float32)[:, -1] / np.float32(rows.shape[1])
+    np.testing.assert_array_equal(m.predict_batch([x])[0], want)

@@ -49,7 +49,10 @@ constexpr int RW_STAGES = 4;
 constexpr int RW_W_BYTES = RW_BN * RW_BK * 4;   // 16 KB: raw W tile; the same again for its remainders
 constexpr int RW_X_BYTES = RW_M * RW_BK * 4;    // 8 KB
 constexpr int RW_STAGE_BYTES = 2 * RW_W_BYTES + 2 * RW_X_BYTES;   // W_raw | W_small | X_raw | X_small = 48 KB
-constexpr int RW_THREADS = 192;                 // warp 0 TMA producer, warp 1 MMA issuer, warps 2-5 converters / epilogue
+// Warp 0 TMA producer, warp 1 MMA issuer, then eight converter warps, two per TMEM lane quadrant, which also bring the
+// partial tile out of tensor memory, a half of its columns each.
+constexpr int RW_CONV = 256;                    // converter threads
+constexpr int RW_THREADS = 64 + RW_CONV;
 constexpr int RW_TMEM_COLS = 256;               // accumulators: big (even k blocks) | big (odd) | small | unused
 constexpr int RW_MAX_CLUSTER = 8;
 constexpr int RW_XCH_BYTES = RW_M * RW_BN * 4;  // exchange area of the reduction: this CTA's partial tile, read by its peers
@@ -161,7 +164,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant
     const uint32_t bar_base = smem_u32(tail);
     auto wfull_bar = [&](int s) { return bar_base + (uint32_t)s * 8u; };                      // TMA landed: raw W tile
     auto xfull_bar = [&](int s) { return bar_base + (uint32_t)(RW_STAGES + s) * 8u; };        // TMA landed: raw X tile
-    auto conv_bar = [&](int s) { return bar_base + (uint32_t)(2 * RW_STAGES + s) * 8u; };     // remainders written (4 warps)
+    auto conv_bar = [&](int s) { return bar_base + (uint32_t)(2 * RW_STAGES + s) * 8u; };     // remainders written (all converter warps)
     auto empty_bar = [&](int s) { return bar_base + (uint32_t)(3 * RW_STAGES + s) * 8u; };    // MMAs of the stage done
     const uint32_t acc_bar = bar_base + (uint32_t)(4 * RW_STAGES) * 8u;                       // all MMAs done
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(tail + 192);
@@ -187,7 +190,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant
         for (int s = 0; s < RW_STAGES; ++s) {
             mbar_init(wfull_bar(s), 1);
             mbar_init(xfull_bar(s), 1);
-            mbar_init(conv_bar(s), 4);
+            mbar_init(conv_bar(s), RW_CONV / 32);
             mbar_init(empty_bar(s), 1);
         }
         mbar_init(acc_bar, 1);
@@ -214,7 +217,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant
     auto convert_w = [&](int s, int ct) {
         const float4* w_raw = reinterpret_cast<const float4*>(smem + (size_t)s * RW_STAGE_BYTES);
         float4* w_small = reinterpret_cast<float4*>(smem + (size_t)s * RW_STAGE_BYTES + RW_W_BYTES);
-        for (int idx = ct; idx < w4; idx += 128) w_small[idx] = tf32_remainder4(w_raw[idx]);
+        for (int idx = ct; idx < w4; idx += RW_CONV) w_small[idx] = tf32_remainder4(w_raw[idx]);
     };
 
     // ---- before the dependency wait: everything that only needs the weights (they are never written) ----
@@ -351,7 +354,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant
         }
     } else {
         // ---------------- converters: remainders of the raw tiles (and the normalisation of X) ----------------
-        const int ct = tid - 64;   // 0..127
+        const int ct = tid - 64;
         bool ok = conv_ok && !*abort_flag;
         for (int i = 0; i < my_nkb && ok; ++i) {
             const int s = i % RW_STAGES;
@@ -366,8 +369,8 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant
             float4* x_small = reinterpret_cast<float4*>(st + 2 * RW_W_BYTES + RW_X_BYTES);
             // X: 64 rows of eight 16-byte chunks; chunk c of row r sits at position c ^ (r & 7) (128-byte swizzle)
 #pragma unroll
-            for (int it = 0; it < (RW_M * 8) / 128; ++it) {
-                const int idx = ct + it * 128;
+            for (int it = 0; it < (RW_M * 8) / RW_CONV; ++it) {
+                const int idx = ct + it * RW_CONV;
                 float4 v = x_raw[idx];
                 if (prm.ln) {
                     const int r = idx >> 3, c = (idx & 7) ^ (r & 7);
@@ -398,8 +401,8 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant
         const int q = warp & 3;                      // the TMEM lane quadrant this warp may read
         const int n_local = q * 32 + lane;
         if (n_local < prm.bn) {
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
+            const int h = (warp - 2) >> 2;           // which half of the rows of X
+            {
                 float v[32];
                 if (ok && my_nkb > 0) {
                     uint32_t b0[32], sm[32];

@@ -1519,7 +1519,7 @@ SplitPlan split_plan(const ConvTcGeom& g, int N) {
     const int tiles[2] = {split_tiles(g, N, 64), split_tiles(g, N, 128)};
     if ((N <= 64 ? tiles[0] : tiles[1]) >= sms) return best;
     const int64_t groups = (k_blocks + TC_GROUP - 1) / TC_GROUP, M = g.B * g.Ho * g.Wo;
-    if (groups > 128 || groups * M * N > SPLIT_MAX_FLOATS) return best;   // 128: sum_parts_kernel's shared memory
+    if (groups > 96 || groups * M * N > SPLIT_MAX_FLOATS) return best;   // 96: sum_parts_kernel's shared memory
     const int whole_tiles = (N <= 64 || tiles[1] * 2 <= sms) ? tiles[0] : tiles[1];
     auto waves = [&](int64_t units) { return (double)((units + sms - 1) / sms); };
     double least = 0.85 * waves(whole_tiles) * (1.5 + 0.55 * k_blocks);   // a split has to be worth its second launch
@@ -1565,11 +1565,11 @@ void launch_conv_tc_parts(const float* in, const ConvTcGeom& g, const float* Wbi
                         al16(e.scale) && al16(e.shift);
     const int64_t M = g.B * g.Ho * g.Wo, total4 = M * N / 4;
     const int groups = (int)((g.win_stride > 0 ? g.kh : g.kh * g.kw * ((g.C + TC_BK - 1) / TC_BK)) + TC_GROUP - 1) / TC_GROUP;
-    // lanes per column: enough loads in flight for few values or many groups
-    const int lanes = total4 >= 148 * 256 && groups <= 16 ? 1 : groups <= 16 ? 4 : 16;
+    // lanes per column: enough threads for the chip, where the values are few by several lanes per column
+    const int lanes = groups <= 16 && total4 >= 148 * 256 ? 1 : groups <= 48 && (total4 >= 148 * 32 || groups <= 8) ? 4 : 16;
     const int cols = 256 / lanes;
     const unsigned grid = (unsigned)std::min<int64_t>((total4 + cols - 1) / cols, 148 * 16);
-    const size_t smem = lanes == 1 ? 0 : (size_t)groups * cols * sizeof(float4);
+    const size_t smem = lanes == 1 ? 0 : (size_t)groups * cols * sizeof(float4);   // at most 48 x 64 or 96 x 16 columns
     ensure(smem <= 48 * 1024, "internal: too many group sums for one block");
     auto kernel = lanes == 1 ? sum_parts_kernel<1> : lanes == 4 ? sum_parts_kernel<4> : sum_parts_kernel<16>;
     launch_pdl(kernel, dim3(grid), dim3(256), smem, s, (const float*)parts, (long long)(M * N), groups, C, (long long)ldc, N / 4, (long long)total4,

@@ -1506,8 +1506,9 @@ __global__ void __launch_bounds__(256) sum_parts_kernel(const float* __restrict_
     }
 }
 
-// Model of the time, in microseconds: a k block of a tile takes 0.55 (one CTA, about 1000 cycles, whatever the tile's
-// width), a work unit 1.5 more; the group sums are written and read once at 4 TB/s, and adding them up is a launch.
+// Model of the time in a chain of launches, in microseconds, from one ResNet-50 image's layers: a launch takes 4 (2 k blocks
+// 5.6, 8 k blocks 8.5 - 9.2, 18 k blocks 13.5), a k block of a tile 0.53 whatever the tile's width, a work unit 0.5 more;
+// adding the group sums up takes 2.5 (4 groups 2.8) and their trip through L2 goes at 5 TB/s.
 struct SplitPlan { int bn = 0, runs = 1, kb_run = 0; };
 SplitPlan split_plan(const ConvTcGeom& g, int N) {
     SplitPlan best;
@@ -1522,12 +1523,12 @@ SplitPlan split_plan(const ConvTcGeom& g, int N) {
     if (groups > 96 || groups * M * N > SPLIT_MAX_FLOATS) return best;   // 96: sum_parts_kernel's shared memory
     const int whole_tiles = (N <= 64 || tiles[1] * 2 <= sms) ? tiles[0] : tiles[1];
     auto waves = [&](int64_t units) { return (double)((units + sms - 1) / sms); };
-    double least = 0.85 * waves(whole_tiles) * (1.5 + 0.55 * k_blocks);   // a split has to be worth its second launch
-    const double sums = 2.5 + 8.0 * (double)groups * (double)M * N / 4e6;
+    double least = 0.93 * (4.0 + waves(whole_tiles) * (0.5 + 0.53 * k_blocks));   // a split has to be worth its second launch
+    const double sums = 6.5 + 8.0 * (double)groups * (double)M * N / 5e6;
     for (int w = 0; w < (N <= 64 ? 1 : 2); ++w)
         for (int run = TC_GROUP; run * 2 <= k_blocks + TC_GROUP - 1; run += TC_GROUP) {
             const int runs = (k_blocks + run - 1) / run;
-            const double t = waves((int64_t)tiles[w] * runs) * (1.5 + 0.55 * run) + sums;
+            const double t = waves((int64_t)tiles[w] * runs) * (0.5 + 0.53 * run) + sums;
             if (t < least) { least = t; best.bn = w ? 128 : 64; best.runs = runs; best.kb_run = run; }
         }
     return best;
@@ -1566,10 +1567,10 @@ void launch_conv_tc_parts(const float* in, const ConvTcGeom& g, const float* Wbi
     const int64_t M = g.B * g.Ho * g.Wo, total4 = M * N / 4;
     const int groups = (int)((g.win_stride > 0 ? g.kh : g.kh * g.kw * ((g.C + TC_BK - 1) / TC_BK)) + TC_GROUP - 1) / TC_GROUP;
     // lanes per column: enough threads for the chip, where the values are few by several lanes per column
-    const int lanes = groups <= 16 && total4 >= 148 * 256 ? 1 : groups <= 48 && (total4 >= 148 * 32 || groups <= 8) ? 4 : 16;
+    const int lanes = groups <= 16 && total4 >= 148 * 256 ? 1 : groups <= 24 && (total4 >= 148 * 32 || groups <= 8) ? 4 : 16;
     const int cols = 256 / lanes;
     const unsigned grid = (unsigned)std::min<int64_t>((total4 + cols - 1) / cols, 148 * 16);
-    const size_t smem = lanes == 1 ? 0 : (size_t)groups * cols * sizeof(float4);   // at most 48 x 64 or 96 x 16 columns
+    const size_t smem = lanes == 1 ? 0 : (size_t)groups * cols * sizeof(float4);   // at most 24 x 64 or 96 x 16 columns
     ensure(smem <= 48 * 1024, "internal: too many group sums for one block");
     auto kernel = lanes == 1 ? sum_parts_kernel<1> : lanes == 4 ? sum_parts_kernel<4> : sum_parts_kernel<16>;
     launch_pdl(kernel, dim3(grid), dim3(256), smem, s, (const float*)parts, (long long)(M * N), groups, C, (long long)ldc, N / 4, (long long)total4,

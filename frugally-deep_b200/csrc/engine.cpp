@@ -889,6 +889,26 @@ struct Exec {
         Epilogue ex;
         ex.bias = wptr(cell_fused ? L.w_cell_bias : L.w_bias);
         gemm(tptr(o.in[0]), F, cell_fused ? L.w_cell_in : L.w_main, L.ldw, X, gu, B * T, gu, (int)F, ex);  // X = in W (+ b)
+        // A few sequences: the whole layer in one launch (gemm_tc.cu; its barrier word is one of the counters in front)
+        if (o.kind == OP_LSTM && !cell_fused && use_tc && !use_skinny && L.act_main.kind == ACT_TANH && L.act_rec.kind == ACT_SIGMOID &&
+            c.w.big_offset[(size_t)L.w_rec] >= 0) {
+            if (float* parts = group_sums(lstm_sequence_floats(B, T, U, L.kdim, wptr(L.w_rec)))) {
+                Rec r;
+                if (prof) {
+                    r = Rec{"gemm", L.name, "tc sequence", nullptr, nullptr, 2.0 * (double)(B * T) * gu * U, B * T, gu, U};
+                    rec_begin(r);
+                }
+                launch_lstm_sequence(c.w.base + c.w.big_offset[(size_t)L.w_rec], c.w.base + c.w.small_offset[(size_t)L.w_rec], L.kdim, X, parts,
+                                     reinterpret_cast<unsigned int*>(c.workspace) + WORKSPACE_COUNTERS - 1, L.flag_b ? tptr(o.out[1]) : nullptr,
+                                     L.flag_b ? tptr(o.out[2]) : nullptr, out, L.flag_a != 0, L.reverse != 0, B, T, U, s);
+                if (prof) {
+                    FDK_CUDA(cudaEventRecord(r.b, s));
+                    prof->push_back(r);
+                }
+                c.launches++;
+                return;
+            }
+        }
         FDK_CUDA(cudaMemsetAsync(h, 0, sizeof(float) * (size_t)(B * U), s));
         FDK_CUDA(cudaMemsetAsync(c2, 0, sizeof(float) * (size_t)(B * U), s));
         float* hc = h;

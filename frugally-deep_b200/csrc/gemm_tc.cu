@@ -1618,6 +1618,275 @@ void launch_lstm_step_tc(const float* h, const float* Wbig, const float* Wsmall,
     launch_tc<128, TC_CELL>(h, gemm_geom(B, U, U), Wbig, Wsmall, ldw, z_unused, (int64_t)4 * U, 4 * U, e, s, &cell);
 }
 
+// ---- all time steps of an LSTM layer on a few sequences in one launch -----------------------------------------
+// A time step of a few rows is a chain, not work: as two launches (group sums, then the cell on them) it took 8.8 us, of
+// which the products are 0.8.  Here the weights stay: CTA (tile, group) keeps the TF32 halves of 128 gate columns x 64 units
+// of h in shared memory (512 units: 16 x 8 CTAs) and per step
+//   multiplies the h of its 64 units (24 MMAs: exactly one accumulator group of gemm_tc_kernel, same operands, same order),
+//   leaves its group sum in L2 and meets all others at ONE grid barrier,
+//   then finishes the cell of its own 64 units for every sequence from the sums of all groups, added in group order.
+// The tiles of a group do that last part redundantly, each with its own copy of c, which is what saves the second barrier
+// and the trip of h through memory; the sums alternate between two buffers, so that nobody overwrites what a slower CTA
+// still reads.  Same bits as the other forms.
+// The CTAs wait for one another: cooperative launch.  Every wait is bounded (TC_WAIT_LIMIT_NS, status word).
+namespace {
+
+constexpr int LQ_ROWS = 8;                    // most sequences: the redundant part grows with them
+constexpr int LQ_THREADS = 256;
+constexpr int LQ_UNITS = TC_GROUP * TC_BK;    // units of h per CTA: one accumulator group
+constexpr int LQ_W_BYTES = TC_GROUP * 2 * 128 * TC_BK * 4;
+constexpr int LQ_SMEM = LQ_W_BYTES + LQ_ROWS * LQ_UNITS * 4 + 64;
+constexpr int LQ_ITEMS = LQ_ROWS * LQ_UNITS / LQ_THREADS;   // cells per thread
+
+struct LstmSeqParams {
+    const float* x;          // gate inputs [B][T][4U] (bias included)
+    float* parts;            // [2][groups][B][4U]
+    unsigned int* arrived;   // grid barrier, zero at launch
+    float* h;                // [B][U] last state, null: not wanted
+    float* c;
+    float* out;              // [B][T][U] (every step) or [B][U] (last step)
+    int B, T, U, groups, every_step, reverse;
+};
+
+__global__ void __launch_bounds__(LQ_THREADS, 1)
+lstm_sequence_kernel(const __grid_constant__ CUtensorMap mapWb, const __grid_constant__ CUtensorMap mapWs, const LstmSeqParams prm) {
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    uint8_t* smem = smem_raw;
+    const uint32_t base = smem_u32(smem_raw);
+    float* hs = reinterpret_cast<float*>(smem + LQ_W_BYTES);                  // [LQ_ROWS][LQ_UNITS]
+    uint8_t* tail = smem + LQ_W_BYTES + LQ_ROWS * LQ_UNITS * 4;
+    const uint32_t w_bar = smem_u32(tail), mma_bar = w_bar + 8u;
+    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(tail + 16);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tail + 20);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int group = (int)blockIdx.x % prm.groups, tile = (int)blockIdx.x / prm.groups;
+    const int n0 = tile * 128, N = 4 * prm.U, U = prm.U, B = prm.B;
+    const int k_blocks = (U + TC_BK - 1) / TC_BK;
+    const int nb = min(TC_GROUP, k_blocks - group * TC_GROUP);
+
+    if (tid == 0) {
+        mbar_init(w_bar, 1);
+        mbar_init(mma_bar, 1);
+        *abort_flag = (base & 1023u) != 0 ? 1 : 0;   // cannot happen: the kernel has no static shared memory
+        if (*abort_flag) atomicCAS(&g_tc_status, 0, 99);
+        fence_barrier_init();
+    }
+    if (warp == 1) {
+        tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), 256u);
+        tmem_relinquish();
+    }
+    for (int i = tid; i < LQ_ROWS * LQ_UNITS; i += LQ_THREADS) hs[i] = 0.0f;   // h and c start at zero
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t a_col = tmem_base + 128u;   // two A slots of 32 + 32 columns behind the accumulator
+    if (tid == 0 && !*abort_flag) {
+        mbar_arrive_expect_tx(w_bar, (uint32_t)(nb * 2 * 128 * TC_BK * 4));
+        for (int b = 0; b < nb; ++b) {
+            const int k = (group * TC_GROUP + b) * TC_BK;
+            tma_load_2d(base + (uint32_t)(b * 32768), &mapWb, k, n0, w_bar);
+            tma_load_2d(base + (uint32_t)(b * 32768 + 16384), &mapWs, k, n0, w_bar);
+        }
+    }
+    float cs[LQ_ITEMS];
+#pragma unroll
+    for (int i = 0; i < LQ_ITEMS; ++i) cs[i] = 0.0f;
+    mbar_wait(w_bar, 0u, abort_flag, 11);
+    __syncthreads();
+    bool ok = !*abort_flag;   // the same for all threads, here and after every grid barrier
+    constexpr uint32_t idesc = make_idesc(TC_BM, 128);
+    const long long gate_pitch = (long long)B * N;
+
+    for (int step = 0; step < prm.T && ok; ++step) {
+        const int t = prm.reverse ? prm.T - 1 - step : step;
+        // ---- h of this CTA's units -> TF32 halves in tensor memory (rows 0 .. 31; the rest of the tile is never read) ----
+        if (warp == 0) {
+#pragma unroll 1
+            for (int b = 0; b < nb; ++b) {
+                uint32_t hi[32], lo[32];
+#pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                    float x[16];
+                    float finite = 0.0f;
+#pragma unroll
+                    for (int k = 0; k < 16; ++k) {
+                        x[k] = lane < LQ_ROWS ? hs[lane * LQ_UNITS + b * TC_BK + half * 16 + k] : 0.0f;
+                        finite = fmaf(x[k], 0.0f, finite);
+                    }
+#pragma unroll
+                    for (int k = 0; k < 16; ++k) {   // the split of gemm_tc_kernel's converters
+                        const uint32_t big = finite == finite ? __float_as_uint(x[k]) & 0xFFFFE000u : rna_tf32(x[k]);
+                        const float rest = x[k] - __uint_as_float(big);
+                        hi[half * 16 + k] = big;
+                        lo[half * 16 + k] = finite == finite ? __float_as_uint(rest) : rna_tf32(rest);
+                    }
+                }
+                const uint32_t dst = a_col + (uint32_t)(b * 2 * TC_BK);
+                tmem_st16(dst, *reinterpret_cast<const uint32_t(*)[16]>(&hi[0]));
+                tmem_st16(dst + 16u, *reinterpret_cast<const uint32_t(*)[16]>(&hi[16]));
+                tmem_st16(dst + (uint32_t)TC_BK, *reinterpret_cast<const uint32_t(*)[16]>(&lo[0]));
+                tmem_st16(dst + (uint32_t)TC_BK + 16u, *reinterpret_cast<const uint32_t(*)[16]>(&lo[16]));
+            }
+            tmem_st_wait();
+        }
+        tc_fence_before();
+        __syncthreads();
+        if (warp == 1) {
+            tc_fence_after();
+            if (lane == 0) {
+                for (int b = 0; b < nb; ++b) {
+                    const uint64_t d = make_smem_desc(base + (uint32_t)(b * 32768));
+                    const uint32_t w_big = (uint32_t)d, w_small = w_big + (16384u >> 4), w_hi = (uint32_t)(d >> 32);
+                    const uint32_t a = a_col + (uint32_t)(b * 2 * TC_BK);
+                    umma_cross8(tmem_base, a, a + (uint32_t)TC_BK, w_big, w_small, w_hi, idesc, b > 0 ? 1u : 0u);
+                    umma_main4(tmem_base, a, w_big, w_hi, idesc);
+                }
+                umma_commit(mma_bar);
+            }
+            __syncwarp();
+        }
+        // this step's gate inputs are fetched while the products run
+        float xv[LQ_ITEMS][4];
+#pragma unroll
+        for (int i = 0; i < LQ_ITEMS; ++i) {
+            const int item = tid + i * LQ_THREADS, b = item / LQ_UNITS, u = group * LQ_UNITS + item % LQ_UNITS;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) xv[i][k] = b < B && u < U ? __ldg(prm.x + ((long long)b * prm.T + t) * N + k * U + u) : 0.0f;
+        }
+        float* parts = prm.parts + (long long)(step & 1) * prm.groups * gate_pitch;
+        if ((warp & 3) == 0) {   // warps 0 and 4 read the accumulator's rows 0 .. 31, half of its columns each
+            mbar_wait(mma_bar, (uint32_t)(step & 1), abort_flag, 12);
+            __syncwarp();
+            tc_fence_after();
+            const int c0 = (warp >> 2) * 64;
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                uint32_t r[32];
+                tmem_ld32(tmem_base + (uint32_t)(c0 + 32 * j), r);
+                tmem_ld_wait();
+                if (lane < B) {
+                    float* dst = parts + (long long)group * gate_pitch + (long long)lane * N + n0 + c0 + 32 * j;
+#pragma unroll
+                    for (int v = 0; v < 8; ++v)
+                        if (n0 + c0 + 32 * j + 4 * v < N)
+                            __stcg(reinterpret_cast<float4*>(dst) + v, make_float4(__uint_as_float(r[4 * v]), __uint_as_float(r[4 * v + 1]),
+                                                                                   __uint_as_float(r[4 * v + 2]), __uint_as_float(r[4 * v + 3])));
+                }
+            }
+            tc_fence_before();
+        }
+        // ---- grid barrier ----
+        __syncthreads();
+        if (tid == 0) {
+            __threadfence();
+            atomicAdd(prm.arrived, 1u);
+            const unsigned int want = (unsigned int)(step + 1) * gridDim.x;
+            unsigned long long t0, t1;
+            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
+            for (unsigned int polls = 1;; ++polls) {
+                unsigned int seen;
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(prm.arrived) : "memory");
+                if (seen >= want) break;
+                if ((polls & 255u) == 0) {
+                    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
+                    if (t1 - t0 > TC_WAIT_LIMIT_NS) {
+                        *abort_flag = 1;
+                        atomicCAS(&g_tc_status, 0, 13);
+                        break;
+                    }
+                }
+            }
+        }
+        __syncthreads();
+        if (*abort_flag) ok = false;
+        // ---- the cells of this CTA's units ----
+        float z[LQ_ITEMS][4];
+#pragma unroll
+        for (int i = 0; i < LQ_ITEMS; ++i) {
+            const int item = tid + i * LQ_THREADS, b = item / LQ_UNITS, u = group * LQ_UNITS + item % LQ_UNITS;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) z[i][k] = 0.0f;
+            if (b >= B || u >= U) continue;
+            const float* p = parts + (long long)b * N + u;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) z[i][k] = __ldcg(p + k * U);
+#pragma unroll 8
+            for (int g = 1; g < prm.groups; ++g)
+#pragma unroll
+                for (int k = 0; k < 4; ++k) z[i][k] += __ldcg(p + g * gate_pitch + k * U);
+        }
+#pragma unroll
+        for (int i = 0; i < LQ_ITEMS; ++i) {
+            const int item = tid + i * LQ_THREADS, b = item / LQ_UNITS, u = group * LQ_UNITS + item % LQ_UNITS;
+            if (b >= B || u >= U) continue;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) z[i][k] = __fadd_rn(__fadd_rn(z[i][k], 0.0f), xv[i][k]);
+            const float cn = __fadd_rn(__fmul_rn(tc_sigmoid(z[i][1]), cs[i]), __fmul_rn(tc_sigmoid(z[i][0]), tanhf(z[i][2])));
+            const float hn = __fmul_rn(tc_sigmoid(z[i][3]), tanhf(cn));
+            cs[i] = cn;
+            hs[item] = hn;
+            if (tile != 0) continue;
+            const bool last = step + 1 == prm.T;
+            if (prm.every_step) prm.out[((long long)b * prm.T + t) * U + u] = hn;
+            else if (last) prm.out[(long long)b * U + u] = hn;
+            if (last && prm.h) {
+                prm.h[(long long)b * U + u] = hn;
+                prm.c[(long long)b * U + u] = cn;
+            }
+        }
+        __syncthreads();
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 1) {
+        tc_fence_after();
+        tmem_dealloc(tmem_base, 256u);
+    }
+}
+
+}  // namespace
+
+int64_t lstm_sequence_floats(int64_t B, int64_t T, int U, int64_t ldw, const void* W) {
+    // one accumulator group per CTA, all of them on the device at once; a single step is no chain
+    if (B < 1 || B > LQ_ROWS || T < 2 || T > (1 << 24) || U < 4 || U % 4 != 0 || U > ldw || (ldw & 3) || (reinterpret_cast<uintptr_t>(W) & 15)) return 0;
+    if (tc_get_encode() == nullptr) return 0;
+    const int64_t tiles = (4 * (int64_t)U + 127) / 128, groups = (U + LQ_UNITS - 1) / LQ_UNITS;
+    return tiles * groups <= tc_sm_count() ? 2 * groups * B * 4 * U : 0;
+}
+
+void launch_lstm_sequence(const float* Wbig, const float* Wsmall, int64_t ldw, const float* x, float* parts, unsigned int* arrived, float* h, float* c,
+                          float* out, bool every_step, bool reverse, int64_t B, int64_t T, int U, cudaStream_t s) {
+    static std::mutex mu;
+    static bool attr_set[64] = {};
+    int dev = 0;
+    FDK_CUDA(cudaGetDevice(&dev));
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        if (dev < 0 || dev >= 64 || !attr_set[dev]) {
+            FDK_CUDA(cudaFuncSetAttribute(lstm_sequence_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LQ_SMEM));
+            if (dev >= 0 && dev < 64) attr_set[dev] = true;
+        }
+    }
+    LstmSeqParams prm;
+    prm.x = x; prm.parts = parts; prm.arrived = arrived; prm.h = h; prm.c = c; prm.out = out;
+    prm.B = (int)B; prm.T = (int)T; prm.U = U; prm.groups = (U + LQ_UNITS - 1) / LQ_UNITS;
+    prm.every_step = every_step ? 1 : 0; prm.reverse = reverse ? 1 : 0;
+    const CUtensorMap mb = tc_make_map_2d(Wbig, 4 * (int64_t)U, U, ldw, 128), ms = tc_make_map_2d(Wsmall, 4 * (int64_t)U, U, ldw, 128);
+    FDK_CUDA(cudaMemsetAsync(arrived, 0, sizeof(unsigned int), s));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)((4 * U + 127) / 128 * prm.groups));
+    cfg.blockDim = dim3(LQ_THREADS);
+    cfg.dynamicSmemBytes = LQ_SMEM;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    FDK_CUDA(cudaLaunchKernelEx(&cfg, lstm_sequence_kernel, mb, ms, prm));
+}
+
 const int* gemm_tc_status_address() {
     int* p = nullptr;
     FDK_CUDA(cudaGetSymbolAddress((void**)&p, g_tc_status));

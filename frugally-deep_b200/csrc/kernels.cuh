@@ -94,6 +94,12 @@ void launch_gemm_tc_parts(const float* A, int64_t lda, const float* Wbig, const 
 // The first kernel alone; returns the number of group sums, [groups][M][N] in `parts`.
 int launch_gemm_tc_group_sums(const float* A, int64_t lda, const float* Wbig, const float* Wsmall, int64_t ldw, int64_t M, int N, int K, float* parts,
                               cudaStream_t s);
+// All time steps of an LSTM layer (tanh / sigmoid) on at most 8 sequences in one launch, results as step by step.  x: gate
+// inputs [B][T][4U], bias included; parts: lstm_sequence_floats floats (0: not this form); arrived: one word of the caller's;
+// h, c: [B][U] last states (both or neither); out: [B][T][U] with every_step, else [B][U].
+int64_t lstm_sequence_floats(int64_t B, int64_t T, int U, int64_t ldw, const void* W);
+void launch_lstm_sequence(const float* Wbig, const float* Wsmall, int64_t ldw, const float* x, float* parts, unsigned int* arrived, float* h, float* c,
+                          float* out, bool every_step, bool reverse, int64_t B, int64_t T, int U, cudaStream_t s);
 // One LSTM time step in one launch: z = h U + x (x = this step's rows of the input product, bias included) never
 // leaves the SM; the epilogue applies the cell (tanh / sigmoid) and writes c in place, the new h to h_next (a buffer
 // other than h: other CTAs still read h) and, if given, to out.  U's rows (and x's columns) must be in the cell order:

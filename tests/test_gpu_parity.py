@@ -1089,10 +1089,11 @@ def test_few_rows_spread_over_the_k_blocks(built_library, side, cin, cout, k, st
     assert launches[0] == launches[1] + 1, f"few rows: {launches[0]} launches, many: {launches[1]}"
 
 
-@pytest.mark.parametrize("units,samples", [(256, 1), (512, 3), (500, 37), (512, 300)])
+@pytest.mark.parametrize("units,samples", [(256, 1), (512, 3), (20, 2), (500, 8), (512, 9), (500, 37), (512, 300)])
 def test_lstm_step_on_group_sums(built_library, units, samples):
     """LSTM steps on few rows: the cell kernel adds the recurrent product's group sums itself; 300 samples run as two chains
-    with a part of the workspace each.  Against the same sequences in a batch whose tiles fill the device, bit for bit."""
+    with a part of the workspace each; at most 8 sequences run all steps in one launch (20 units: a partial tile and one k
+    block; 500: a partial k block).  Against the same sequences in a batch whose tiles fill the device, bit for bit."""
     rng = np.random.default_rng(units + samples)
     T, F = 5, 12
     b = mw.ModelBuilder("m")

@@ -1453,16 +1453,30 @@ __global__ void __launch_bounds__(256) sum_parts_kernel(const float* __restrict_
         if (L == 1) {
             if (i < total4) {
                 v = __ldcg(p + i);
-#pragma unroll 8
-                for (int g = 1; g < groups; ++g) {
-                    const float4 t = __ldcg(p + (long long)g * pitch4 + i);
-                    v.x += t.x; v.y += t.y; v.z += t.z; v.w += t.w;
+                // eight loads in flight at a time, also where fewer are left (a plain unrolled loop walks its remainder alone)
+#pragma unroll 1
+                for (int g0 = 1; g0 < groups; g0 += 8) {
+                    float4 t[8];
+#pragma unroll
+                    for (int k = 0; k < 8; ++k)
+                        if (g0 + k < groups) t[k] = __ldcg(p + (long long)(g0 + k) * pitch4 + i);
+#pragma unroll
+                    for (int k = 0; k < 8; ++k)
+                        if (g0 + k < groups) { v.x += t[k].x; v.y += t[k].y; v.z += t[k].z; v.w += t[k].w; }
                 }
             }
         } else {
             if (i < total4) {
-#pragma unroll 8
-                for (int g = l; g < groups; g += L) sp_sum[g * COLS + col] = __ldcg(p + (long long)g * pitch4 + i);
+#pragma unroll 1
+                for (int g0 = l; g0 < groups; g0 += 6 * L) {
+                    float4 t[6];
+#pragma unroll
+                    for (int k = 0; k < 6; ++k)
+                        if (g0 + k * L < groups) t[k] = __ldcg(p + (long long)(g0 + k * L) * pitch4 + i);
+#pragma unroll
+                    for (int k = 0; k < 6; ++k)
+                        if (g0 + k * L < groups) sp_sum[(g0 + k * L) * COLS + col] = t[k];
+                }
             }
             __syncthreads();
             if (l == 0 && i < total4) {
@@ -1634,6 +1648,7 @@ namespace {
 constexpr int LQ_ROWS = 8;                    // most sequences: the redundant part grows with them
 constexpr int LQ_THREADS = 256;
 constexpr int LQ_UNITS = TC_GROUP * TC_BK;    // units of h per CTA: one accumulator group
+constexpr int LQ_GROUPS = 8;                  // most groups: 512 units (more would not fit the SMs but for a few sizes)
 constexpr int LQ_W_BYTES = TC_GROUP * 2 * 128 * TC_BK * 4;
 constexpr int LQ_SMEM = LQ_W_BYTES + LQ_ROWS * LQ_UNITS * 4 + 64;
 constexpr int LQ_ITEMS = LQ_ROWS * LQ_UNITS / LQ_THREADS;   // cells per thread
@@ -1809,12 +1824,19 @@ lstm_sequence_kernel(const __grid_constant__ CUtensorMap mapWb, const __grid_con
             for (int k = 0; k < 4; ++k) z[i][k] = 0.0f;
             if (b >= B || u >= U) continue;
             const float* p = parts + (long long)b * N + u;
+            float v[LQ_GROUPS][4];   // all in flight before the first add
 #pragma unroll
-            for (int k = 0; k < 4; ++k) z[i][k] = __ldcg(p + k * U);
-#pragma unroll 8
-            for (int g = 1; g < prm.groups; ++g)
+            for (int g = 0; g < LQ_GROUPS; ++g)
+                if (g < prm.groups) {
 #pragma unroll
-                for (int k = 0; k < 4; ++k) z[i][k] += __ldcg(p + g * gate_pitch + k * U);
+                    for (int k = 0; k < 4; ++k) v[g][k] = __ldcg(p + g * gate_pitch + k * U);
+                }
+#pragma unroll
+            for (int g = 0; g < LQ_GROUPS; ++g)
+                if (g < prm.groups) {
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) z[i][k] = g == 0 ? v[0][k] : z[i][k] + v[g][k];
+                }
         }
 #pragma unroll
         for (int i = 0; i < LQ_ITEMS; ++i) {
@@ -1852,7 +1874,7 @@ int64_t lstm_sequence_floats(int64_t B, int64_t T, int U, int64_t ldw, const voi
     if (B < 1 || B > LQ_ROWS || T < 2 || T > (1 << 24) || U < 4 || U % 4 != 0 || U > ldw || (ldw & 3) || (reinterpret_cast<uintptr_t>(W) & 15)) return 0;
     if (tc_get_encode() == nullptr) return 0;
     const int64_t tiles = (4 * (int64_t)U + 127) / 128, groups = (U + LQ_UNITS - 1) / LQ_UNITS;
-    return tiles * groups <= tc_sm_count() ? 2 * groups * B * 4 * U : 0;
+    return groups <= LQ_GROUPS && tiles * groups <= tc_sm_count() ? 2 * groups * B * 4 * U : 0;
 }
 
 void launch_lstm_sequence(const float* Wbig, const float* Wsmall, int64_t ldw, const float* x, float* parts, unsigned int* arrived, float* h, float* c,

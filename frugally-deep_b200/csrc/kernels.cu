@@ -1493,10 +1493,21 @@ __global__ void __launch_bounds__(64) lstm_cell_parts_kernel(const float* __rest
         const float cv = __ldcg(c + i);
 #pragma unroll
         for (int k = 0; k < 4; ++k) z[k] = __ldcg(p + k * U);
-#pragma unroll 8
-        for (int g = 1; g < groups; ++g) {
+#pragma unroll 1
+        for (int g0 = 1; g0 < groups; g0 += 8) {   // the loads of eight groups in flight, also where fewer are left
+            float v[8][4];
 #pragma unroll
-            for (int k = 0; k < 4; ++k) z[k] += __ldcg(p + g * pitch + k * U);
+            for (int g = 0; g < 8; ++g)
+                if (g0 + g < groups) {
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) v[g][k] = __ldcg(p + (g0 + g) * pitch + k * U);
+                }
+#pragma unroll
+            for (int g = 0; g < 8; ++g)
+                if (g0 + g < groups) {
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) z[k] += v[g][k];
+                }
         }
 #pragma unroll
         for (int k = 0; k < 4; ++k) z[k] = __fadd_rn(__fadd_rn(z[k], 0.0f), xv[k]);

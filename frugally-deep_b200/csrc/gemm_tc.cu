@@ -1642,7 +1642,8 @@ void launch_lstm_step_tc(const float* h, const float* Wbig, const float* Wsmall,
 // The tiles of a group do that last part redundantly, each with its own copy of c, which is what saves the second barrier
 // and the trip of h through memory; the sums alternate between two buffers, so that nobody overwrites what a slower CTA
 // still reads.  Same bits as the other forms.  Two layers of 512 units, 3 sequences of 120 steps: 2134 -> 1284 us, 5.1 us a
-// step.  At most 8 sequences: the sums that every CTA reads grow with them (a step of 8 moves 8 MB through L2).
+// step; 8 sequences 1572 us, where 9, as two launches a step, take 1910.  At most 8: the sums that every CTA reads grow with
+// them (a step of 8 moves 8 MB through L2).
 // The CTAs wait for one another: cooperative launch.  Every wait is bounded (TC_WAIT_LIMIT_NS, status word).
 namespace {
 

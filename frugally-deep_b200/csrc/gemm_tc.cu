@@ -272,9 +272,24 @@ struct TcParams {
 // none; they come from the warp's parameter block in shared memory), residual and clipping are warp-uniform
 // branches.  (Specialising this by template made the kernel several hundred KB of code and instruction
 // fetch its bottleneck.)
+//
+// The last step (clip): a ReLU, or (top) a ReLU with a finite maximum `hi` in act_apply's meaning (threshold 0, slope 0;
+// relu_layer.hpp:40-46), which keeps NaN and makes NaN of -inf (0 * -inf) where a min / max pair alone turns both into 0.
+// Values go in pairs and both forms share all but one packed FMA (a loop of its own for either form: ResNet-50 on one
+// image 610 -> 637 us, instruction fetch; this way 623 -> 611 with the values of sum_parts_kernel kept out of local memory).
+__device__ __forceinline__ void clip_pair(float& a, float& b, float hi, bool top) {   // hi = inf without top
+    float wa, wb;
+    asm("min.NaN.f32 %0, %1, %2;" : "=f"(wa) : "f"(a), "f"(hi));
+    asm("min.NaN.f32 %0, %1, %2;" : "=f"(wb) : "f"(b), "f"(hi));
+    a = fmaxf(0.0f, wa);
+    b = fmaxf(0.0f, wb);
+    if (top)
+        asm("{\n .reg .b64 r, w, z;\n mov.b64 r, {%0, %1};\n mov.b64 w, {%2, %3};\n mov.b64 z, {%4, %4};\n fma.rn.f32x2 r, w, z, r;\n"
+            " mov.b64 {%0, %1}, r;\n}" : "+f"(a), "+f"(b) : "f"(wa), "f"(wb), "f"(0.0f));
+}
 template <int CPT, int J0>
 __device__ __forceinline__ void epi_block(const float (&sum)[CPT], const float* __restrict__ wprm, uint8_t* __restrict__ row_ptr, int lane,
-                                          bool has_res, bool clip, float lo, float hi) {
+                                          bool has_res, bool clip, bool top, float hi) {
     // In phases, every phase's shared-memory loads ahead of its arithmetic and all stores last, so that no load
     // has to wait behind a store it might alias.
     float v[32];
@@ -305,7 +320,7 @@ __device__ __forceinline__ void epi_block(const float (&sum)[CPT], const float* 
     }
     if (clip) {
 #pragma unroll
-        for (int t = 0; t < 32; ++t) v[t] = fminf(fmaxf(lo, v[t]), hi);
+        for (int t = 0; t < 32; t += 2) clip_pair(v[t], v[t + 1], hi, top);
     }
 #pragma unroll
     for (int c = 0; c < 8; ++c)
@@ -331,7 +346,7 @@ __device__ __forceinline__ void tc_sts4(uint32_t addr, float4 v) {
     asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
 }
 __device__ __forceinline__ void epi_block_direct(uint32_t taddr, uint32_t wprm_s, uint32_t prm_stride, uint32_t row_s, int lane, bool has_res,
-                                                 bool clip, float lo, float hi) {
+                                                 bool clip, bool top, float hi) {
     const uint32_t sw = (uint32_t)(lane & 7);
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
@@ -355,8 +370,8 @@ __device__ __forceinline__ void epi_block_direct(uint32_t taddr, uint32_t wprm_s
             v[2] = __fadd_rn(__fmul_rn(v[2], ps[k].z), pt[k].z); v[3] = __fadd_rn(__fmul_rn(v[3], ps[k].w), pt[k].w);
             if (has_res) { v[0] += pr[k].x; v[1] += pr[k].y; v[2] += pr[k].z; v[3] += pr[k].w; }
             if (clip) {
-#pragma unroll
-                for (int t = 0; t < 4; ++t) v[t] = fminf(fmaxf(lo, v[t]), hi);
+                clip_pair(v[0], v[1], hi, top);
+                clip_pair(v[2], v[3], hi, top);
             }
             tc_sts4(row_s + ((((uint32_t)(4 * i + k)) ^ sw) << 4), make_float4(v[0], v[1], v[2], v[3]));
         }
@@ -655,10 +670,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
         uint32_t acc_phase = 0;
         bool ok = true;
         const bool has_res = prm.epi.residual != nullptr;
-        // final activation of the TMA epilogue: none, ReLU, or ReLU clipped at max_value (threshold 0, slope 0)
-        const bool clip = prm.epi.act2.kind != ACT_NONE;
-        const float clip_lo = 0.0f;
-        const float clip_hi = prm.epi.act2.kind == ACT_RELU_GEN ? prm.epi.act2.p0 : __int_as_float(0x7f800000);
+        // final activation of the TMA epilogue (fused_activation)
+        const bool clip = prm.epi.act2.kind != ACT_NONE, clip_top = prm.epi.act2.kind == ACT_RELU_GEN;
+        const float clip_hi = clip_top ? prm.epi.act2.p0 : __int_as_float(0x7f800000);
         constexpr int NSUB = CPT / 32;                    // 32-column blocks per lane and tile
         const int ew = warp - TC_EPI_WARP0;
         const int nbuf = prm.nbuf;                        // staging buffers of this warp (power of two)
@@ -828,7 +842,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
                     }
                     const uint32_t row_s = stg_addr + (uint32_t)(b * Cfg::STG_BUF_BYTES + lane * 128);
                     epi_block_direct(taddr0 + 32u * (uint32_t)j, wprm_s + (uint32_t)(32 * j * 4), (uint32_t)(CPT * 4), row_s, lane, has_res, clip,
-                                     clip_lo, clip_hi);
+                                     clip_top, clip_hi);
                     if (j == g.nsub - 1) {   // the last read of the accumulator set is done
                         tc_fence_before();
                         __syncwarp();
@@ -944,8 +958,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
                     if (!mbar_wait(res_bar(ew, b), (res_phase >> b) & 1u, abort_flag, 6)) { ok = false; break; }
                     res_phase ^= 1u << b;
                     uint8_t* buf = stg_buf + b * Cfg::STG_BUF_BYTES;
-                    if (j == 0) epi_block<CPT, 0>(sum, wprm, buf + lane * 128, lane, true, false, 0.f, 0.f);
-                    else epi_block<CPT, (NSUB > 1 ? 32 : 0)>(sum, wprm, buf + lane * 128, lane, true, false, 0.f, 0.f);
+                    if (j == 0) epi_block<CPT, 0>(sum, wprm, buf + lane * 128, lane, true, false, false, 0.f);
+                    else epi_block<CPT, (NSUB > 1 ? 32 : 0)>(sum, wprm, buf + lane * 128, lane, true, false, false, 0.f);
                 }
                 if (!ok) break;
                 const long long srow = (long long)g.qb + lane;
@@ -986,8 +1000,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
                         __syncwarp();
                         ring = (ring + 1) & (nbuf - 1);
                     }
-                    if (j == 0) epi_block<CPT, 0>(sum, wprm, buf + lane * 128, lane, has_res, clip, clip_lo, clip_hi);
-                    else epi_block<CPT, (NSUB > 1 ? 32 : 0)>(sum, wprm, buf + lane * 128, lane, has_res, clip, clip_lo, clip_hi);
+                    if (j == 0) epi_block<CPT, 0>(sum, wprm, buf + lane * 128, lane, has_res, clip, clip_top, clip_hi);
+                    else epi_block<CPT, (NSUB > 1 ? 32 : 0)>(sum, wprm, buf + lane * 128, lane, has_res, clip, clip_top, clip_hi);
                     fence_proxy_async();
                     __syncwarp();
                     if (lane == 0) {
@@ -1259,6 +1273,13 @@ struct CellState {
     int U = 0;
 };
 
+// Last activations that the epilogue through shared memory and TMA knows: none, ReLU, and a ReLU with a maximum (finite, not
+// negative; slope 0, threshold 0).
+bool fused_activation(const ActSpec& a) {
+    return a.kind == ACT_NONE || a.kind == ACT_RELU ||
+           (a.kind == ACT_RELU_GEN && a.p0 >= 0.0f && a.p0 <= FLT_MAX && a.p1 == 0.0f && a.p2 == 0.0f);
+}
+
 struct PartsOut {
     float* base = nullptr;
     int runs = 1, kb_run = 0;
@@ -1308,9 +1329,7 @@ void launch_tc(const float* in, const ConvTcGeom& g, const float* Wb, const floa
         prm.sx = 1; prm.dx = 1; prm.dy = 1; prm.pad_t = 0; prm.pad_l = 0;
     }
     // Epilogue through TMA when the rows of the output (and of the residual) start on 16-byte boundaries.
-    const bool plain_act = e.act1.kind == ACT_NONE &&
-                           (e.act2.kind == ACT_NONE || e.act2.kind == ACT_RELU ||
-                            (e.act2.kind == ACT_RELU_GEN && e.act2.p1 == 0.0f && e.act2.p2 == 0.0f));  // clipped ReLU: slope 0, threshold 0
+    const bool plain_act = e.act1.kind == ACT_NONE && fused_activation(e.act2);
     const bool spread = g.out_sx > 0;  // output pixels are not dense
     prm.out_sx = spread ? g.out_sx : ldc;
     prm.out_sy = spread ? g.out_sy : (long long)g.Wo * ldc;
@@ -1492,8 +1511,8 @@ __global__ void __launch_bounds__(256) sum_parts_kernel(const float* __restrict_
         if (l == 0 && i < total4) {
             const long long row = i / n4;
             const int n = (int)(i - row * n4) * 4;
-            float o[4] = {v.x, v.y, v.z, v.w};
             if (aligned) {
+                float o[4] = {v.x, v.y, v.z, v.w};
                 // the form of the epilogue through TMA: absent parameters are 0, 1, 0
                 const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
                 const float4 b = e.bias ? __ldg(reinterpret_cast<const float4*>(e.bias + n)) : z4;
@@ -1507,12 +1526,14 @@ __global__ void __launch_bounds__(256) sum_parts_kernel(const float* __restrict_
                     o[0] += r.x; o[1] += r.y; o[2] += r.z; o[3] += r.w;
                 }
                 if (e.act2.kind != ACT_NONE) {
-                    const float hi = e.act2.kind == ACT_RELU_GEN ? e.act2.p0 : __int_as_float(0x7f800000);
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) o[k] = fminf(fmaxf(0.0f, o[k]), hi);
+                    const bool top = e.act2.kind == ACT_RELU_GEN;
+                    const float hi = top ? e.act2.p0 : __int_as_float(0x7f800000);
+                    clip_pair(o[0], o[1], hi, top);
+                    clip_pair(o[2], o[3], hi, top);
                 }
                 *reinterpret_cast<float4*>(C + row * ldc + n) = make_float4(o[0], o[1], o[2], o[3]);
             } else {
+                const float o[4] = {v.x, v.y, v.z, v.w};   // (of its own: the loop's index puts it into local memory)
 #pragma unroll 1
                 for (int k = 0; k < 4; ++k) C[row * ldc + n + k] = epi_apply(e, o[k], row, n + k);
             }
@@ -1573,8 +1594,7 @@ void launch_conv_tc_parts(const float* in, const ConvTcGeom& g, const float* Wbi
     launch_parts(in, g, Wbig, Wsmall, ldw, N, plan, parts, s);
     Epilogue e = epilogue;
     if (e.scale == nullptr && e.residual == nullptr && e.act2.none()) std::swap(e.act1, e.act2);
-    const bool plain_act = e.act1.kind == ACT_NONE &&
-                           (e.act2.kind == ACT_NONE || e.act2.kind == ACT_RELU || (e.act2.kind == ACT_RELU_GEN && e.act2.p1 == 0.0f && e.act2.p2 == 0.0f));
+    const bool plain_act = e.act1.kind == ACT_NONE && fused_activation(e.act2);
     auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
     const int aligned = plain_act && (ldc & 3) == 0 && al16(C) && (e.residual == nullptr || ((e.ldr & 3) == 0 && al16(e.residual))) && al16(e.bias) &&
                         al16(e.scale) && al16(e.shift);

@@ -1146,3 +1146,30 @@ def test_global_pooling_tiles(built_library, side, channels, kind):
     rows = x.reshape(5, -1, channels)
     want = rows.max(axis=1) if "Max" in kind else np.cumsum(rows, axis=1, dtype=np.float32)[:, -1] / np.float32(rows.shape[1])
     np.testing.assert_array_equal(m.predict_batch([x])[0], want)
+
+
+@pytest.mark.parametrize("tail", ["relu6", "relu max", "bn relu max"])
+@pytest.mark.parametrize("cin,cout,n", [(32, 64, 1), (300, 64, 2), (300, 64, 1300), (300, 66, 2)])
+def test_clipped_relu_keeps_what_is_not_a_number(built_library, cin, cout, n, tail):
+    """A ReLU with a maximum behind a product, in each form of the epilogue (one accumulator group; group sums of few rows; whole
+    products of several groups; odd columns): NaN stays NaN, -inf gives NaN (0 * -inf, relu_layer.hpp:40-46), +inf the maximum."""
+    rng = np.random.default_rng(cin + cout)
+    b = mw.ModelBuilder("m")
+    i = b.input([4, 4, cin])
+    bias = rng.normal(scale=4, size=cout).astype(np.float32)
+    bias[[0, 7, 33]], bias[[1, 13, 40]], bias[[2, 20, 63]] = np.nan, np.inf, -np.inf
+    y = mw.conv2d(b, i, "c", rng.normal(size=(1, 1, cin, cout)).astype(np.float32) / np.sqrt(cin), bias,
+                  activation="relu6" if tail == "relu6" else "linear")
+    if tail == "bn relu max":
+        y = mw.batch_norm(b, y, "bn", rng.normal(size=cout).astype(np.float32), rng.uniform(0.5, 2, cout).astype(np.float32),
+                          rng.uniform(0.5, 2, cout).astype(np.float32), rng.normal(size=cout).astype(np.float32))
+    if tail != "relu6":
+        y = mw.relu(b, y, "relu", max_value=2.5)
+    text = model_text(b.to_json([y], [[4, 4, cout]]))
+    x = rng.normal(size=(n, 4, 4, cin)).astype(np.float32)
+    got = fdeep_b200.read_model_from_string(text, verify=False).predict_batch([x])[0]
+    for s in {0, n - 1}:
+        want = oracle_outputs(text, [[x[s]]])[0][0]
+        np.testing.assert_array_equal(np.isnan(got[s]), np.isnan(want))
+        # sums of 300 products of size 1 / sqrt(300), through a factor of at most 2 / sqrt(0.5): far below 1e-5
+        np.testing.assert_allclose(got[s], want, rtol=1e-5, atol=1e-5)

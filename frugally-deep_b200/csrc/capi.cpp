@@ -180,6 +180,7 @@ int fdk_model_sync(fdk_model* m, int device_index) {
         ensure(m != nullptr, "null model");
         ensure(device_index >= 0 && device_index < m->eng->num_devices(), "invalid device index");
         DeviceCtx& c = m->eng->ctx(device_index);
+        std::lock_guard<std::mutex> lk(c.sync_mu);   // one at a time: they share the word the flag is copied to
         int prev = 0;
         FDK_CUDA(cudaGetDevice(&prev));
         FDK_CUDA(cudaSetDevice(c.device));

@@ -58,6 +58,7 @@ Engine::Engine(LoadedModel&& lm, const std::vector<int>& devices, const EngineOp
         DeviceGuard g(d);
         FDK_CUDA(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
         FDK_CUDA(cudaStreamCreateWithFlags(&c->copy_stream, cudaStreamNonBlocking));
+        FDK_CUDA(cudaStreamCreateWithFlags(&c->record_stream, cudaStreamNonBlocking));
         FDK_CUDA(cudaStreamCreateWithFlags(&c->aux_stream, cudaStreamNonBlocking));
         FDK_CUDA(cudaEventCreateWithFlags(&c->fork_event, cudaEventDisableTiming));
         FDK_CUDA(cudaEventCreateWithFlags(&c->join_event, cudaEventDisableTiming));
@@ -93,6 +94,7 @@ Engine::~Engine() {
         cudaFreeHost(c->h_err);
         cudaStreamDestroy(c->stream);
         if (c->copy_stream) cudaStreamDestroy(c->copy_stream);
+        if (c->record_stream) cudaStreamDestroy(c->record_stream);
         if (c->aux_stream) { cudaStreamSynchronize(c->aux_stream); cudaStreamDestroy(c->aux_stream); }
         if (c->fork_event) cudaEventDestroy(c->fork_event);
         if (c->join_event) cudaEventDestroy(c->join_event);
@@ -1323,14 +1325,14 @@ void Engine::replay(DeviceCtx& c, const Plan& p, int64_t batch, std::vector<cons
     if (!r->exec && !r->unusable) {
         const int64_t before = c.launches;
         cudaGraph_t graph = nullptr;
-        FDK_CUDA(cudaStreamBeginCapture(c.stream, cudaStreamCaptureModeRelaxed));
+        FDK_CUDA(cudaStreamBeginCapture(c.record_stream, cudaStreamCaptureModeRelaxed));
         bool ok = true;
         try {
-            queue(c.stream);
+            queue(c.record_stream);
         } catch (const std::exception&) {
             ok = false;
         }
-        ok = cudaStreamEndCapture(c.stream, &graph) == cudaSuccess && ok && graph != nullptr;
+        ok = cudaStreamEndCapture(c.record_stream, &graph) == cudaSuccess && ok && graph != nullptr;
         ok = ok && cudaGraphInstantiate(&r->exec, graph, 0) == cudaSuccess;
         if (graph) cudaGraphDestroy(graph);
         r->launches = c.launches - before;

@@ -94,6 +94,7 @@ struct DeviceCtx {
     int device = 0;
     cudaStream_t stream = nullptr;
     cudaStream_t copy_stream = nullptr;  // host-to-device copies of the chunks of a large block
+    cudaStream_t record_stream = nullptr;  // only ever captured (Engine::replay): other threads may wait for `stream` meanwhile
     // second chain of a recurrent layer on a large batch (forked from and joined to the stream of the call)
     cudaStream_t aux_stream = nullptr;
     cudaEvent_t fork_event = nullptr, join_event = nullptr;
@@ -117,6 +118,7 @@ struct DeviceCtx {
     std::vector<RecordedCall> calls;   // see Engine::replay
     uint64_t call_clock = 0;
     std::mutex mu;                 // held while a call queues its work on this device
+    std::mutex sync_mu;            // held by fdk_model_sync (h_err[0])
     // Order between calls that use the arena / workspace from different streams: the last use recorded `busy` on
     // `busy_stream`; the next use on another stream waits for it (Engine::order_after_last_use / mark_use).
     cudaEvent_t busy = nullptr;

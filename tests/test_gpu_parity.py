@@ -1173,3 +1173,46 @@ def test_clipped_relu_keeps_what_is_not_a_number(built_library, cin, cout, n, ta
         np.testing.assert_array_equal(np.isnan(got[s]), np.isnan(want))
         # sums of 300 products of size 1 / sqrt(300), through a factor of at most 2 / sqrt(0.5): far below 1e-5
         np.testing.assert_allclose(got[s], want, rtol=1e-5, atol=1e-5)
+
+
+def test_sync_while_another_thread_records(built_library):
+    """Two threads make device calls of ever new sizes on one model, the second call of each being recorded, and wait with sync();
+    a third waits all the time.  Nobody gets an error and every result is that of a call on its own."""
+    import threading
+    import torch
+    m, _ = load(mw.build_small_cnn(), True)
+    alone, _ = load(mw.build_small_cnn(), True)
+    sizes = list(range(1, 41))
+    x = np.random.default_rng(11).random((max(sizes) + 2, 32, 32, 3), dtype=np.float32)
+    want = alone.predict_batch([x])[0]
+    errors, done = [], threading.Event()
+
+    def caller(t):
+        try:
+            d_in = torch.from_numpy(x).cuda()
+            d_out = torch.zeros((len(x), 10), device="cuda")
+            torch.cuda.synchronize()
+            for n in sizes[t::2]:
+                for rep in range(4):
+                    m.predict_batch_device([d_in[rep % 3:].data_ptr()], [[32, 32, 3]], n, [d_out.data_ptr()])
+                    m.sync()
+                    np.testing.assert_array_equal(d_out[:n].cpu().numpy(), want[rep % 3:rep % 3 + n], err_msg=f"{n} samples, call {rep}")
+        except BaseException as e:
+            errors.append(e)
+
+    def waiter():
+        try:
+            while not done.is_set():
+                m.sync()
+        except BaseException as e:
+            errors.append(e)
+
+    threads = [threading.Thread(target=caller, args=(t,)) for t in range(2)]
+    w = threading.Thread(target=waiter)
+    for th in threads + [w]:
+        th.start()
+    for th in threads:
+        th.join()
+    done.set()
+    w.join()
+    assert not errors, errors[0]

@@ -1139,22 +1139,35 @@ struct Exec {
 };
 }  // namespace
 
-// The caller's memory takes the place of an output's buffer in the arena when it can: the buffer holds exactly that output
-// (not a part, not an input handed through), the memory is aligned as the kernels' vector and TMA stores want it, and it is
-// none of the call's inputs.
-static bool bound_output(const Plan& p, size_t o, const float* d_out, int64_t batch, const float* const* d_in) {
-    for (size_t i = 0; i < p.inputs.size(); ++i)
-        if (d_out && d_in[i] < d_out + batch * p.tensors[(size_t)p.outputs[o]].shape.volume() && d_out < d_in[i] + batch * p.in_shapes[i].volume()) return false;
-    const TensorInfo& t = p.tensors[(size_t)p.outputs[o]];
-    const BufferInfo& b = p.buffers[(size_t)t.buf];
-    if (!d_out || b.ext_input >= 0 || b.elems != t.shape.volume() || (reinterpret_cast<uintptr_t>(d_out) & 255) != 0) return false;
-    for (size_t k = 0; k < o; ++k)
-        if (p.tensors[(size_t)p.outputs[k]].buf == t.buf) return false;   // the first of several views
-    return true;
+// Which outputs their kernels write into the caller's memory instead of the arena, per plan output: that memory or null.  It
+// has to be memory of this device (a copy reaches other GPUs and the host as well, a kernel's store need not), aligned as
+// the kernels' vector and TMA stores want it, and apart from every input and every other output of the call, because the
+// plan's operations read it like any buffer; and the buffer has to hold exactly that output (not a part, not an input handed
+// through, the first of several views).
+static std::vector<float*> bind_outputs(const DeviceCtx& c, const Plan& p, int64_t batch, const float* const* d_in, float* const* d_out) {
+    std::vector<float*> bound(p.outputs.size(), nullptr);
+    auto floats = [&](size_t o) { return batch * p.tensors[(size_t)p.outputs[o]].shape.volume(); };
+    auto apart = [](const float* a, int64_t na, const float* b, int64_t nb) { return a + na <= b || b + nb <= a; };
+    for (size_t o = 0; o < p.outputs.size(); ++o) {
+        const TensorInfo& t = p.tensors[(size_t)p.outputs[o]];
+        const BufferInfo& b = p.buffers[(size_t)t.buf];
+        if (!d_out[o] || b.ext_input >= 0 || b.elems != t.shape.volume() || (reinterpret_cast<uintptr_t>(d_out[o]) & 255) != 0) continue;
+        bool ok = true;
+        for (size_t k = 0; k < o; ++k) ok = ok && p.tensors[(size_t)p.outputs[k]].buf != t.buf;
+        for (size_t k = 0; k < p.outputs.size(); ++k) ok = ok && (k == o || !d_out[k] || apart(d_out[o], floats(o), d_out[k], floats(k)));
+        for (size_t i = 0; i < p.inputs.size(); ++i) ok = ok && apart(d_out[o], floats(o), d_in[i], batch * p.in_shapes[i].volume());
+        cudaPointerAttributes at;
+        if (ok && cudaPointerGetAttributes(&at, d_out[o]) != cudaSuccess) {
+            cudaGetLastError();
+            ok = false;
+        }
+        if (ok && at.type == cudaMemoryTypeDevice && at.device == c.device) bound[o] = d_out[o];
+    }
+    return bound;
 }
 
 void Engine::execute(DeviceCtx& c, const Plan& p, int64_t B, const float* const* d_in, cudaStream_t s, std::string* profile, const KvCache* kv,
-                     const std::vector<char>* wanted, float* const* d_out, int* err) {
+                     const std::vector<char>* wanted, const std::vector<float*>* bound, int* err) {
     ensure_arena(c, std::max<int64_t>(p.arena_elems, 64) * B);
     Exec ex{*this, c, p, B, d_in, s, opt_.use_tc};
     ex.use_skinny = opt_.skinny;
@@ -1162,10 +1175,10 @@ void Engine::execute(DeviceCtx& c, const Plan& p, int64_t B, const float* const*
     ex.kv = kv;
     ex.wanted = wanted;
     ex.err = err ? err : c.d_err;
-    if (d_out) {
+    if (bound) {
         ex.bound.assign(p.buffers.size(), nullptr);
         for (size_t o = 0; o < p.outputs.size(); ++o)
-            if (bound_output(p, o, d_out[o], B, d_in)) ex.bound[(size_t)p.tensors[(size_t)p.outputs[o]].buf] = d_out[o];
+            if ((*bound)[o]) ex.bound[(size_t)p.tensors[(size_t)p.outputs[o]].buf] = (*bound)[o];
     }
     std::vector<Exec::Rec> recs;
     if (profile) ex.prof = &recs;
@@ -1232,15 +1245,16 @@ void Engine::predict_batch_device(int dev_index, int64_t batch, const float* con
     std::vector<char> wanted(p->outputs.size(), 1);
     for (size_t o = 0; o < p->outputs.size(); ++o) wanted[o] = d_out[o] != nullptr ? 1 : 0;
     auto queue = [&](cudaStream_t on) {
-        execute(c, *p, batch, d_in, on, profile, kv, &wanted, d_out);
+        const std::vector<float*> bound = bind_outputs(c, *p, batch, d_in, d_out);
+        execute(c, *p, batch, d_in, on, profile, kv, &wanted, &bound);
         for (size_t o = 0; o < p->outputs.size(); ++o) {
-            if (!d_out[o] || bound_output(*p, o, d_out[o], batch, d_in)) continue;  // output not wanted, or written by its kernel
+            if (!d_out[o] || bound[o]) continue;  // output not wanted, or written by its kernel
             const TensorInfo& t = p->tensors[(size_t)p->outputs[o]];
             const BufferInfo& b = p->buffers[(size_t)t.buf];
             const float* src = b.ext_input >= 0 ? d_in[b.ext_input] : c.arena + b.offset * batch;
             for (size_t k = 0; k < o; ++k)   // another view of an output that lives in the caller's memory
-                if (p->tensors[(size_t)p->outputs[k]].buf == t.buf && bound_output(*p, k, d_out[k], batch, d_in)) src = d_out[k];
-            FDK_CUDA(cudaMemcpyAsync(d_out[o], src, sizeof(float) * (size_t)(batch * t.shape.volume()), cudaMemcpyDeviceToDevice, on));
+                if (p->tensors[(size_t)p->outputs[k]].buf == t.buf && bound[k]) src = bound[k];
+            FDK_CUDA(cudaMemcpyAsync(d_out[o], src, sizeof(float) * (size_t)(batch * t.shape.volume()), cudaMemcpyDefault, on));
         }
     };
     // A small call is replayed on memory of the engine, one copy in and one out per tensor: what is recorded knows nothing of

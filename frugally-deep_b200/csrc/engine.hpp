@@ -229,10 +229,10 @@ private:
     std::shared_ptr<Plan> get_plan(const std::vector<TShape>& in_shapes);
     std::shared_ptr<Plan> compile(const std::vector<TShape>& in_shapes);
     // wanted (optional, per plan output): 0 = the caller does not read this output, so it need not be computed.
-    // d_out (optional, per plan output): where the caller wants it; set entries have to be copied there afterwards only if
-    // `bound_output` says that the producing kernel cannot write there itself.  err: flag of the device-side input checks.
+    // bound (optional, per plan output): memory that the producing kernel writes instead of the arena, or null.  err: flag of the
+    // device-side input checks.
     void execute(DeviceCtx& c, const Plan& p, int64_t B, const float* const* d_in, cudaStream_t s, std::string* profile = nullptr,
-                 const KvCache* kv = nullptr, const std::vector<char>* wanted = nullptr, float* const* d_out = nullptr, int* err = nullptr);
+                 const KvCache* kv = nullptr, const std::vector<char>* wanted = nullptr, const std::vector<float*>* bound = nullptr, int* err = nullptr);
     void ensure_arena(DeviceCtx& c, int64_t elems);
     // Runs `queue(stream)` or replays what it launched before (see RecordedCall); call with c.mu held.
     template <typename F>

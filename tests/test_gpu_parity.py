@@ -1216,3 +1216,36 @@ def test_sync_while_another_thread_records(built_library):
     done.set()
     w.join()
     assert not errors, errors[0]
+
+
+@pytest.mark.parametrize("n", [3, 700])
+def test_outputs_that_share_memory_or_lie_on_the_host(built_library, n):
+    """Device calls, staged (3 samples) and not (700): where two outputs share memory the later one ends up there, computed
+    from an intact earlier one; outputs in page-locked host memory and in memory of the GPU are alike."""
+    import torch
+    rng = np.random.default_rng(5)
+    b = mw.ModelBuilder("m")
+    i = b.input([12, 12, 8])
+    y = mw.conv2d(b, i, "a", rng.normal(size=(3, 3, 8, 16)).astype(np.float32), rng.normal(size=16).astype(np.float32), padding="same")
+    z = mw.conv2d(b, y, "b", rng.normal(size=(3, 3, 16, 16)).astype(np.float32) / 12, rng.normal(size=16).astype(np.float32), padding="same")
+    m = fdeep_b200.read_model_from_string(model_text(b.to_json([y, z], [[12, 12, 16]] * 2)), verify=False)
+    x = torch.from_numpy(rng.normal(size=(n, 12, 12, 8)).astype(np.float32)).cuda()
+
+    def call(a, c):
+        torch.cuda.synchronize()
+        m.predict_batch_device([x.data_ptr()], [[12, 12, 8]], n, [a.data_ptr(), c.data_ptr()])
+        m.sync()
+        return a.cpu().numpy(), c.cpu().numpy()
+
+    def new(**where):
+        return torch.zeros((n, 12, 12, 16), **where)
+
+    want = call(new(device="cuda"), new(device="cuda"))
+    for rep in range(3):
+        shift = n // 2   # the later output starts in the middle of the earlier one, which is read after its first tiles are written
+        both = torch.zeros((n + shift, 12, 12, 16), device="cuda")
+        np.testing.assert_array_equal(call(both[:n], both[shift:])[1], want[1])
+        np.testing.assert_array_equal(both[:shift].cpu().numpy(), want[0][:shift])
+        got = call(new(pin_memory=True), new(pin_memory=True))
+        np.testing.assert_array_equal(got[0], want[0])
+        np.testing.assert_array_equal(got[1], want[1])

@@ -65,6 +65,7 @@ Engine::Engine(LoadedModel&& lm, const std::vector<int>& devices, const EngineOp
         FDK_CUDA(cudaEventCreateWithFlags(&c->busy, cudaEventDisableTiming));
         FDK_CUDA(cudaMalloc(&c->d_err, 2 * sizeof(int)));
         FDK_CUDA(cudaMemset(c->d_err, 0, 2 * sizeof(int)));
+        FDK_CUDA(cudaMalloc(&c->grid_barrier, sizeof(unsigned int)));
         FDK_CUDA(cudaMallocHost(&c->h_err, 8 * sizeof(int)));
         std::memset(c->h_err, 0, 8 * sizeof(int));
         c->status[0] = gemm_tc_status_address();
@@ -88,6 +89,8 @@ Engine::~Engine() {
         cudaFree(c->device_stage);
         cudaFree(c->byte_stage);
         cudaFree(c->workspace);
+        for (auto& sums : c->sums) sums.release([](float* p) { cudaFree(p); });
+        cudaFree(c->grid_barrier);
         cudaFree(c->d_err);
         cudaFreeHost(c->h_in);
         cudaFreeHost(c->h_out);
@@ -363,37 +366,33 @@ struct Exec {
     // The workspace may move when it grows (a recorded graph that holds the old address must be recorded again: the
     // decode session compares addresses before every replay).
     void ensure_workspace(int64_t ws) {
-        ensure(try_workspace(ws), "device workspace allocation of " + std::to_string(ws * 4) + " bytes failed");
-    }
-    // Group sums of products of few rows (gemm_tc.cu) live behind the arrival counters, one part per chain of time steps
-    // (their products run side by side).  Null: not wanted (floats = 0), or no memory for it, and the product runs whole.
-    static constexpr int64_t WORKSPACE_COUNTERS = 1024;
-    int chain = 0;               // which part this product uses
-    int64_t chain_floats = 0;    // size of the first chain's part while two chains run (-1: no memory for both), else 0
-    float* group_sums(int64_t floats) {
-        if (floats <= 0 || chain_floats < 0) return nullptr;
-        const int64_t first = WORKSPACE_COUNTERS + (chain ? chain_floats : 0);
-        if (!try_workspace(first + floats)) return nullptr;
-        return c.workspace + first;
-    }
-    bool try_workspace(int64_t ws) {
-        if (ws <= c.workspace_elems) return true;
-        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-        FDK_CUDA(cudaStreamIsCapturing(s, &cap));
-        if (cap != cudaStreamCaptureStatusNone) return false;   // nothing may be allocated here
+        if (ws <= c.workspace_elems) return;
         FDK_CUDA(cudaStreamSynchronize(s));
         if (c.aux_stream) FDK_CUDA(cudaStreamSynchronize(c.aux_stream));
         if (c.busy_valid) FDK_CUDA(cudaEventSynchronize(c.busy));
         if (c.workspace) FDK_CUDA(cudaFree(c.workspace));
         c.workspace = nullptr; c.workspace_elems = 0;
-        if (cudaMalloc(&c.workspace, sizeof(float) * (size_t)ws) != cudaSuccess) {
-            cudaGetLastError();
-            c.workspace = nullptr;
-            return false;
-        }
-        FDK_CUDA(cudaMemset(c.workspace, 0, sizeof(float) * (size_t)ws));  // the arrival counters start at zero (synchronous)
+        FDK_CUDA(cudaMalloc(&c.workspace, sizeof(float) * (size_t)ws));
+        // the arrival counters start at zero; waited for, because the next use may be on another stream (cudaMemset itself may
+        // return before it is done, on a stream that orders nothing here)
+        FDK_CUDA(cudaMemsetAsync(c.workspace, 0, sizeof(float) * (size_t)ws, s));
+        FDK_CUDA(cudaStreamSynchronize(s));
         c.workspace_elems = ws;
-        return true;
+    }
+    // Memory for the group sums of a product of few rows (gemm_tc.cu), one block per chain of time steps (their products run
+    // side by side); needs no clearing and never moves.  Null: not wanted (floats = 0), or there is none, or it would have
+    // to be allocated while the stream is captured; the product then runs whole.
+    int chain = 0;
+    float* group_sums(int64_t floats) {
+        if (floats <= 0) return nullptr;
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        FDK_CUDA(cudaStreamIsCapturing(s, &cap));
+        return c.sums[chain].get(floats, cap == cudaStreamCaptureStatusNone, [](int64_t n) {
+            float* p = nullptr;
+            if (cudaMalloc(&p, sizeof(float) * (size_t)n) == cudaSuccess) return p;
+            cudaGetLastError();
+            return (float*)nullptr;
+        });
     }
     // Query, key and value projections of one attention block on the same rows: one launch of the skinny kernel when
     // all three qualify for it (same shape, bias-only epilogues).  Returns false when nothing was launched.
@@ -891,7 +890,7 @@ struct Exec {
         Epilogue ex;
         ex.bias = wptr(cell_fused ? L.w_cell_bias : L.w_bias);
         gemm(tptr(o.in[0]), F, cell_fused ? L.w_cell_in : L.w_main, L.ldw, X, gu, B * T, gu, (int)F, ex);  // X = in W (+ b)
-        // A few sequences: the whole layer in one launch (gemm_tc.cu; its barrier word is one of the counters in front)
+        // A few sequences: the whole layer in one launch (gemm_tc.cu)
         if (o.kind == OP_LSTM && !cell_fused && use_tc && !use_skinny && L.act_main.kind == ACT_TANH && L.act_rec.kind == ACT_SIGMOID &&
             c.w.big_offset[(size_t)L.w_rec] >= 0) {
             if (float* parts = group_sums(lstm_sequence_floats(B, T, U, L.kdim, wptr(L.w_rec)))) {
@@ -901,8 +900,7 @@ struct Exec {
                     rec_begin(r);
                 }
                 launch_lstm_sequence(c.w.base + c.w.big_offset[(size_t)L.w_rec], c.w.base + c.w.small_offset[(size_t)L.w_rec], L.kdim, X, parts,
-                                     reinterpret_cast<unsigned int*>(c.workspace) + WORKSPACE_COUNTERS - 1, L.flag_b ? tptr(o.out[1]) : nullptr,
-                                     L.flag_b ? tptr(o.out[2]) : nullptr, out, L.flag_a != 0, L.reverse != 0, B, T, U, s);
+                                     c.grid_barrier, L.flag_b ? tptr(o.out[1]) : nullptr, L.flag_b ? tptr(o.out[2]) : nullptr, out, L.flag_a != 0, L.reverse != 0, B, T, U, s);
                 if (prof) {
                     FDK_CUDA(cudaEventRecord(r.b, s));
                     prof->push_back(r);
@@ -999,16 +997,6 @@ struct Exec {
         // the batch they are computed in, so the split cannot change them.
         const bool two_chains = prof == nullptr && B >= 256 && c.aux_stream != nullptr && c.aux_stream != s;
         const int64_t first_rows = two_chains ? (B / 2 + 127) / 128 * 128 : B;
-        struct ChainParts {   // both chains' group sums, in place before the first launch
-            int64_t& floats;
-            ~ChainParts() { floats = 0; }
-        } chain_parts{chain_floats};
-        if (two_chains) {
-            auto most = [&](int64_t nb) { return std::max(gemm_tc_parts_floats(nb, gu, U), gemm_tc_parts_floats(nb, U, U)); };
-            chain_floats = std::max(most(first_rows), gemm_tc_parts_floats(first_rows, 2 * U, U));
-            const int64_t second = std::max(most(B - first_rows), gemm_tc_parts_floats(B - first_rows, 2 * U, U));
-            if (chain_floats + second > 0 && !try_workspace(WORKSPACE_COUNTERS + chain_floats + second)) chain_floats = -1;
-        }
         cudaStream_t main_stream = s;
         if (two_chains) {
             FDK_CUDA(cudaEventRecord(c.fork_event, main_stream));

@@ -7,6 +7,7 @@
 #pragma once
 
 #include "common.hpp"
+#include "growing_memory.hpp"
 #include "model.hpp"
 
 #include <map>
@@ -78,7 +79,7 @@ struct DeviceWeights {
 struct RecordedCall {
     const Plan* plan = nullptr;
     int64_t batch = 0;
-    std::vector<const void*> where;    // staging buffers, arena, workspace
+    std::vector<const void*> where;    // staging buffers, arena, workspace (group sums never move)
     float low = 0.f, high = 0.f;
     cudaGraphExec_t exec = nullptr;
     int64_t launches = 0;
@@ -110,6 +111,8 @@ struct DeviceCtx {
     int64_t h_out_elems = 0;
     float* workspace = nullptr;    // partial tiles of split-K products
     int64_t workspace_elems = 0;
+    GrowingMemory sums[2];         // group sums of products of few rows, one per chain of time steps (recorded launches keep its addresses)
+    unsigned int* grid_barrier = nullptr;   // word of the LSTM sequence kernel's barrier (zeroed before each launch)
     // Input checks on the device (embedding range, ...): [0] for calls that leave work in flight (read by fdk_model_sync),
     // [1] for host calls, cleared by the kernel that ends each of them.
     int* d_err = nullptr;

@@ -1249,3 +1249,25 @@ def test_outputs_that_share_memory_or_lie_on_the_host(built_library, n):
         got = call(new(pin_memory=True), new(pin_memory=True))
         np.testing.assert_array_equal(got[0], want[0])
         np.testing.assert_array_equal(got[1], want[1])
+
+
+def test_a_callers_graph_outlives_other_batches(built_library):
+    """A device call on a few samples, captured by the caller, still gives its results after calls of other sizes, each of which
+    needs more memory for the group sums of its products (and less of the other buffers than the first, large call)."""
+    import torch
+    m, _ = load(mw.build_resnet50(size=64, width=32, classes=10, top="linear"), True)
+    alone, _ = load(mw.build_resnet50(size=64, width=32, classes=10, top="linear"), True)
+    x = mw.inputs_resnet50(64, size=64)
+    m.predict_batch([x])
+    m.predict_batch([x[:1]])
+    d_in, d_out = torch.from_numpy(x[:1]).cuda(), torch.zeros((1, 10), device="cuda")
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, capture_error_mode="relaxed"):
+        m.predict_batch_device([d_in.data_ptr()], [[64, 64, 3]], 1, [d_out.data_ptr()], stream=torch.cuda.current_stream().cuda_stream)
+    for n in (3, 7, 20):
+        m.predict_batch([x[:n]])
+    for s in range(4):
+        d_in.copy_(torch.from_numpy(x[s:s + 1]))
+        graph.replay()
+        torch.cuda.synchronize()
+        np.testing.assert_array_equal(d_out.cpu().numpy(), alone.predict_batch([x[s:s + 1]])[0])

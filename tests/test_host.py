@@ -256,3 +256,22 @@ def test_plan_of_conv_lstm(built_library):
         js, x, wants = conv_lstm_case(**case)
         txt = fdeep_b200.plan_describe(model_text(js), [list(x.shape)])
         assert txt.count("convlstm_cell") == case["T"], txt
+
+
+def run_host_program(name, tmp_path, flags=()):
+    """Compiles tests/cpp/<name>.cpp against the library's headers, runs it and expects "ok"."""
+    import shutil
+    import subprocess
+    if shutil.which("g++") is None:
+        pytest.skip("no host compiler")
+    exe = str(tmp_path / name)
+    cmd = ["g++", "-std=c++17", "-O1", "-I", os.path.join(ROOT, "frugally-deep_b200", "csrc"), os.path.join(ROOT, "tests", "cpp", name + ".cpp"),
+           "-o", exe, *flags]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    r = subprocess.run([exe], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0 and r.stdout.startswith("ok"), (r.returncode, r.stdout + r.stderr)
+
+
+def test_growing_memory(tmp_path):
+    run_host_program("growing_memory", tmp_path)

@@ -189,6 +189,7 @@ void Engine::ensure_arena(DeviceCtx& c, int64_t elems) {
     if (c.arena) FDK_CUDA(cudaFree(c.arena));
     c.arena = nullptr;
     c.arena_elems = 0;
+    c.memory_moves++;
     const cudaError_t e = cudaMalloc(&c.arena, (size_t)elems * sizeof(float));
     if (e != cudaSuccess) {
         cudaGetLastError();
@@ -364,14 +365,14 @@ struct Exec {
     }
 
     // The workspace may move when it grows (a recorded graph that holds the old address must be recorded again: the
-    // decode session compares addresses before every replay).
+    // decode session checks memory_moves before every replay).
     void ensure_workspace(int64_t ws) {
         if (ws <= c.workspace_elems) return;
         FDK_CUDA(cudaStreamSynchronize(s));
         if (c.aux_stream) FDK_CUDA(cudaStreamSynchronize(c.aux_stream));
         if (c.busy_valid) FDK_CUDA(cudaEventSynchronize(c.busy));
         if (c.workspace) FDK_CUDA(cudaFree(c.workspace));
-        c.workspace = nullptr; c.workspace_elems = 0;
+        c.workspace = nullptr; c.workspace_elems = 0; c.memory_moves++;
         FDK_CUDA(cudaMalloc(&c.workspace, sizeof(float) * (size_t)ws));
         // the arrival counters start at zero; waited for, because the next use may be on another stream (cudaMemset itself may
         // return before it is done, on a stream that orders nothing here)
@@ -1280,7 +1281,7 @@ void Engine::predict_batch_device(int dev_index, int64_t batch, const float* con
         float* const* caller_out = d_out;
         d_in = st_in.data();
         d_out = st_out.data();
-        replay(c, *p, batch, std::move(where), 0.f, 0.f, s, queue);
+        replay(c, *p, batch, std::move(where), false, 0.f, 0.f, s, queue);
         d_in = caller_in;
         d_out = caller_out;
         for (size_t o = 0; o < p->outputs.size(); ++o)
@@ -1297,7 +1298,7 @@ void Engine::predict_batch_device(int dev_index, int64_t batch, const float* con
 // addresses of the staging buffers, the arena and the workspace belong to the key because other calls may make them move.
 // No address of the caller's is ever part of a recording.
 template <typename F>
-void Engine::replay(DeviceCtx& c, const Plan& p, int64_t batch, std::vector<const void*> where, float low, float high, cudaStream_t s, F&& queue) {
+void Engine::replay(DeviceCtx& c, const Plan& p, int64_t batch, std::vector<const void*> where, bool host, float low, float high, cudaStream_t s, F&& queue) {
     static const bool enabled = [] { const char* v = getenv("FDK_PREDICT_GRAPH"); return !(v && *v == '0'); }();
     if (!enabled) {
         queue(s);
@@ -1305,12 +1306,13 @@ void Engine::replay(DeviceCtx& c, const Plan& p, int64_t batch, std::vector<cons
     }
     where.push_back(c.arena);
     where.push_back(c.workspace);
+    const uint64_t memory = c.memory_moves, staging = host ? c.staging_moves : 0;
     RecordedCall* r = nullptr;
     for (auto& k : c.calls)
-        if (k.plan == &p && k.batch == batch && k.low == low && k.high == high && k.where == where) r = &k;
+        if (k.plan == &p && k.batch == batch && k.memory == memory && k.staging == staging && k.low == low && k.high == high && k.where == where) r = &k;
     if (!r) {
         queue(s);
-        if (where[where.size() - 2] != c.arena || where.back() != c.workspace) return;   // they moved: not this kind's steady state yet
+        if (memory != c.memory_moves) return;   // they moved: not this kind's steady state yet
         if (c.calls.size() >= 32) {
             auto oldest = std::min_element(c.calls.begin(), c.calls.end(), [](const RecordedCall& x, const RecordedCall& y) { return x.last_use < y.last_use; });
             if (oldest->exec) cudaGraphExecDestroy(oldest->exec);
@@ -1318,6 +1320,7 @@ void Engine::replay(DeviceCtx& c, const Plan& p, int64_t batch, std::vector<cons
         }
         RecordedCall k;
         k.plan = &p; k.batch = batch; k.low = low; k.high = high;
+        k.memory = memory; k.staging = staging;
         k.where = std::move(where);
         k.last_use = ++c.call_clock;
         c.calls.push_back(std::move(k));
@@ -1390,14 +1393,14 @@ void Engine::run_block(DeviceCtx& c, const Plan& p, const std::vector<int64_t>& 
         if (c.h_in_elems < nb * in_total) {
             FDK_CUDA(cudaStreamSynchronize(c.stream));
             if (c.h_in) FDK_CUDA(cudaFreeHost(c.h_in));
-            c.h_in = nullptr; c.h_in_elems = 0;
+            c.h_in = nullptr; c.h_in_elems = 0; c.staging_moves++;
             FDK_CUDA(cudaMallocHost(&c.h_in, sizeof(float) * (size_t)(nb * in_total)));
             c.h_in_elems = nb * in_total;
         }
         if (c.in_stage_elems < nb * in_total) {
             FDK_CUDA(cudaStreamSynchronize(c.stream));
             if (c.in_stage) FDK_CUDA(cudaFree(c.in_stage));
-            c.in_stage = nullptr; c.in_stage_elems = 0;
+            c.in_stage = nullptr; c.in_stage_elems = 0; c.staging_moves++;
             FDK_CUDA(cudaMalloc(&c.in_stage, sizeof(float) * (size_t)(nb * in_total)));
             c.in_stage_elems = nb * in_total;
         }
@@ -1405,14 +1408,14 @@ void Engine::run_block(DeviceCtx& c, const Plan& p, const std::vector<int64_t>& 
             FDK_CUDA(cudaStreamSynchronize(c.stream));
             FDK_CUDA(cudaStreamSynchronize(c.copy_stream));
             if (c.byte_stage) FDK_CUDA(cudaFree(c.byte_stage));
-            c.byte_stage = nullptr; c.byte_stage_bytes = 0;
+            c.byte_stage = nullptr; c.byte_stage_bytes = 0; c.staging_moves++;
             FDK_CUDA(cudaMalloc(&c.byte_stage, (size_t)(nb * in_total)));
             c.byte_stage_bytes = nb * in_total;
         }
         if (c.h_out_elems < nb * out_total) {
             FDK_CUDA(cudaStreamSynchronize(c.stream));
             if (c.h_out) FDK_CUDA(cudaFreeHost(c.h_out));
-            c.h_out = nullptr; c.h_out_elems = 0;
+            c.h_out = nullptr; c.h_out_elems = 0; c.staging_moves++;
             FDK_CUDA(cudaMallocHost(&c.h_out, sizeof(float) * (size_t)(nb * out_total)));
             c.h_out_elems = nb * out_total;
         }
@@ -1581,7 +1584,7 @@ void Engine::run_block(DeviceCtx& c, const Plan& p, const std::vector<int64_t>& 
                 for (size_t o = 0; o < n_out; ++o) same_addresses = same_addresses && !direct[o];
                 if (same_addresses) {
                     std::vector<const void*> where = {c.in_stage, c.h_in, c.h_out, bytes ? (const void*)c.byte_stage : nullptr, tiny ? (const void*)c.h_err : nullptr};
-                    replay(c, p, cnb, std::move(where), bytes ? bytes->low : 0.f, bytes ? bytes->high : 0.f, c.stream, queue);
+                    replay(c, p, cnb, std::move(where), true, bytes ? bytes->low : 0.f, bytes ? bytes->high : 0.f, c.stream, queue);
                 } else {
                     queue(c.stream);
                 }

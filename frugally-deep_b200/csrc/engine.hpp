@@ -74,12 +74,13 @@ struct DeviceWeights {
     std::vector<int64_t> small_offset;  // TF32 low halves or -1
 };
 
-// The launches of one call, recorded as a CUDA graph: everything that fixes them is in the key (the plan, the batch and every
-// address the launches hold).
+// The launches of one call, recorded as a CUDA graph: everything that fixes them is in the key (the plan, the batch, every
+// address the launches hold, and how often those buffers have been replaced).
 struct RecordedCall {
     const Plan* plan = nullptr;
     int64_t batch = 0;
     std::vector<const void*> where;    // staging buffers, arena, workspace (group sums never move)
+    uint64_t memory = 0, staging = 0;  // DeviceCtx::memory_moves / staging_moves (a smaller buffer may come to lie at an old address)
     float low = 0.f, high = 0.f;
     cudaGraphExec_t exec = nullptr;
     int64_t launches = 0;
@@ -120,6 +121,8 @@ struct DeviceCtx {
     const int* status[3] = {nullptr, nullptr, nullptr};   // device addresses of the contraction and tile kernels' status words
     std::vector<RecordedCall> calls;   // see Engine::replay
     uint64_t call_clock = 0;
+    uint64_t memory_moves = 0;     // times the arena or the workspace was given back
+    uint64_t staging_moves = 0;    // the same of the staging buffers of host calls
     std::mutex mu;                 // held while a call queues its work on this device
     std::mutex sync_mu;            // held by fdk_model_sync (h_err[0])
     // Order between calls that use the arena / workspace from different streams: the last use recorded `busy` on
@@ -237,9 +240,10 @@ private:
     void execute(DeviceCtx& c, const Plan& p, int64_t B, const float* const* d_in, cudaStream_t s, std::string* profile = nullptr,
                  const KvCache* kv = nullptr, const std::vector<char>* wanted = nullptr, const std::vector<float*>* bound = nullptr, int* err = nullptr);
     void ensure_arena(DeviceCtx& c, int64_t elems);
-    // Runs `queue(stream)` or replays what it launched before (see RecordedCall); call with c.mu held.
+    // Runs `queue(stream)` or replays what it launched before (see RecordedCall); call with c.mu held.  host: the launches use
+    // the staging buffers of host calls.
     template <typename F>
-    void replay(DeviceCtx& c, const Plan& p, int64_t batch, std::vector<const void*> where, float low, float high, cudaStream_t s, F&& queue);
+    void replay(DeviceCtx& c, const Plan& p, int64_t batch, std::vector<const void*> where, bool host, float low, float high, cudaStream_t s, F&& queue);
     void run_block(DeviceCtx& c, const Plan& p, const std::vector<int64_t>& sample_ids, const float* const* in_ptrs,
                    float* const* out_ptrs, const ByteScale* bytes = nullptr);
     void upload_weights(DeviceCtx& c);

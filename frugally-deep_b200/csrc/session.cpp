@@ -173,7 +173,7 @@ void DecodeSession::step(const float* tokens, float* next_tokens, float* logits)
 bool DecodeSession::replay_position() {
     DeviceCtx& c = step_.ctx(0);
     std::lock_guard<std::mutex> lk(c.mu);
-    if (c.arena != graph_arena_ || c.workspace != graph_workspace_) return false;
+    if (c.memory_moves != graph_moves_) return false;
     step_.order_after_last_use(c, stream_);
     FDK_CUDA(cudaGraphLaunch(graph_exec_, stream_));
     step_.mark_use(c, stream_);
@@ -207,6 +207,10 @@ void DecodeSession::step_impl(const float* tokens, float* next_tokens, float* lo
         } else if (use_graph_ && warmed_) {
             // second and later positions of this kind: every buffer has its final size, record the launches
             const int64_t l0 = c.launches;
+            {
+                std::lock_guard<std::mutex> lk(c.mu);
+                graph_moves_ = c.memory_moves;
+            }
             cudaGraph_t graph = nullptr;
             FDK_CUDA(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeRelaxed));
             bool ok = true;
@@ -221,8 +225,6 @@ void DecodeSession::step_impl(const float* tokens, float* next_tokens, float* lo
             bool replayed = false;
             const bool recorded = ok && ce == cudaSuccess && graph && cudaGraphInstantiate(&graph_exec_, graph, 0) == cudaSuccess;
             if (recorded) {
-                graph_arena_ = c.arena;
-                graph_workspace_ = c.workspace;
                 graph_launches_ = c.launches - l0;
                 c.launches = l0;
                 replayed = replay_position();

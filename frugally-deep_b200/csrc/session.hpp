@@ -73,8 +73,7 @@ private:
     int* d_len_ = nullptr;           // rows in the cache, as the kernels see it
     bool device_len_ = true, use_graph_ = true, warmed_ = false;
     cudaGraphExec_t graph_exec_ = nullptr;
-    const void* graph_arena_ = nullptr;      // addresses the recorded launches hold
-    const void* graph_workspace_ = nullptr;
+    uint64_t graph_moves_ = 0;               // DeviceCtx::memory_moves when it was recorded
     int64_t graph_launches_ = 0;
     double t_plan_ = 0, t_queue_ = 0, t_wait_ = 0;  // host seconds, accumulated when FDK_SESSION_TIMING is set
     double t_device_ = 0;                            // device milliseconds between the first and the last launch of a position

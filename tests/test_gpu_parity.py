@@ -1271,3 +1271,28 @@ def test_a_callers_graph_outlives_other_batches(built_library):
         graph.replay()
         torch.cuda.synchronize()
         np.testing.assert_array_equal(d_out.cpu().numpy(), alone.predict_batch([x[s:s + 1]])[0])
+
+
+def test_recorded_calls_forget_memory_that_was_given_back(built_library):
+    """A call whose buffers cannot be had gives the old ones back; the next small call gets small ones, possibly at the old
+    address.  What was recorded on the large ones must not be launched on them."""
+    import torch
+    m, _ = load(mw.build_small_cnn(), True)
+    alone, _ = load(mw.build_small_cnn(), True)
+    x = mw.inputs_small_cnn(200)
+    want = alone.predict_batch([x])[0]
+    d_in, d_out = torch.from_numpy(x).cuda(), torch.zeros((200, 10), device="cuda")
+    torch.cuda.synchronize()
+
+    def call(n):
+        m.predict_batch_device([d_in.data_ptr()], [[32, 32, 3]], n, [d_out.data_ptr()])
+        m.sync()
+        np.testing.assert_array_equal(d_out[:n].cpu().numpy(), want[:n])
+
+    for rep in range(3):
+        for _ in range(3):
+            call(200)
+        with pytest.raises(fdeep_b200.FdeepError, match="arena allocation"):
+            m.predict_batch_device([d_in.data_ptr()], [[32, 32, 3]], 10 ** 8, [d_out.data_ptr()])   # terabytes
+        call(1)
+        call(200)

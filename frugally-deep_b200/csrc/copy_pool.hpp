@@ -1,12 +1,18 @@
-// A few host threads that copy memory together: what moves a caller's pageable or scattered samples into page-locked staging
-// memory (one thread copies about 10 GB/s, the bus takes five times that).  One job at a time; a caller that finds the pool
-// busy copies by itself.  Started on first use, at most 7 threads, joined when the process ends.
+// Host threads that copy memory together: what moves a caller's pageable or scattered samples into page-locked staging memory
+// (one thread copies about 10 GB/s, the bus takes five times that).  Several callers (one per device) may have a copy under
+// way; up to 7 threads are started for each of them, no more than half of the cores in all, and every thread takes parts
+// from the copies in turn.  A caller takes parts of its own copy as well, so that it gets done whatever the threads do, also
+// where none could be started or (in a forked child) none exists.
 #pragma once
+
+#include <unistd.h>
 
 #include <algorithm>
 #include <condition_variable>
-#include <cstdint>
+#include <deque>
+#include <exception>
 #include <functional>
+#include <memory>
 #include <mutex>
 #include <thread>
 #include <vector>
@@ -15,73 +21,89 @@ namespace fdk {
 
 class CopyPool {
 public:
-    static CopyPool& instance() {
-        static CopyPool pool;
-        return pool;
+    static constexpr int PARTS = 8;
+    // The pool of the process; its threads end with the last of its users.
+    static std::shared_ptr<CopyPool> shared() {
+        static std::mutex mu;
+        static std::weak_ptr<CopyPool> known;
+        std::lock_guard<std::mutex> lk(mu);
+        std::shared_ptr<CopyPool> p = known.lock();
+        if (!p) known = p = std::make_shared<CopyPool>(std::max(0, (int)std::thread::hardware_concurrency() / 2 - 1));
+        return p;
     }
-    // job(part, parts) for every part in 0 .. parts - 1, in parallel; returns when all are done.  The jobs must not throw.
+    explicit CopyPool(int most_threads) : s_(std::make_unique<State>()) { s_->most = most_threads; }
+    CopyPool(const CopyPool&) = delete;
+    CopyPool& operator=(const CopyPool&) = delete;
+    ~CopyPool() {
+        if (getpid() != pid_) {
+            s_.release();   // a forked child: the threads are the parent's; nothing here can be joined or waited out
+            return;
+        }
+        {
+            std::lock_guard<std::mutex> lk(s_->mu);
+            s_->stop = true;
+        }
+        s_->wake.notify_all();
+        for (auto& t : s_->workers) t.join();
+    }
+    // job(part, PARTS) for every part, side by side; returns when all are done.  The job must not throw.
     void run(const std::function<void(int, int)>& job) {
-        std::unique_lock<std::mutex> use(use_, std::try_to_lock);
-        if (!use.owns_lock() || workers_.empty()) {
+        if (getpid() != pid_) {
             job(0, 1);
             return;
         }
-        const int parts = (int)workers_.size() + 1;
-        {
-            std::lock_guard<std::mutex> lk(mu_);
-            job_ = &job;
-            parts_ = parts;
-            left_ = parts - 1;
-            ++round_;
+        State& s = *s_;
+        Copy own{&job};
+        std::unique_lock<std::mutex> lk(s.mu);
+        s.copies.push_back(&own);
+        ++s.active;
+        while ((int)s.workers.size() < std::min(s.most, (PARTS - 1) * s.active)) {
+            try {
+                s.workers.emplace_back([&s] { s.work(); });
+            } catch (const std::exception&) {
+                s.most = (int)s.workers.size();   // no more threads to be had
+            }
         }
-        wake_.notify_all();
-        job(parts - 1, parts);
-        std::unique_lock<std::mutex> lk(mu_);
-        done_.wait(lk, [&] { return left_ == 0; });
-        job_ = nullptr;
+        s.wake.notify_all();
+        while (own.next < PARTS) s.take(lk, own);
+        s.done.wait(lk, [&] { return own.done == PARTS; });
+        --s.active;
     }
 
 private:
-    CopyPool() {
-        const int cores = (int)std::thread::hardware_concurrency();
-        const int n = std::min(7, std::max(0, cores / 2 - 1));
-        for (int i = 0; i < n; ++i) workers_.emplace_back([this, i] { work(i); });
-    }
-    ~CopyPool() {
-        {
-            std::lock_guard<std::mutex> lk(mu_);
-            stop_ = true;
+    struct Copy {
+        const std::function<void(int, int)>* job;
+        int next = 0, done = 0;
+    };
+    struct State {
+        int most = 0;
+        int active = 0;
+        bool stop = false;
+        std::mutex mu;
+        std::condition_variable wake, done;
+        std::deque<Copy*> copies;   // those with parts left
+        std::vector<std::thread> workers;
+        // One part of a copy that has parts left; mu is held on entry and on return.
+        void take(std::unique_lock<std::mutex>& lk, Copy& c) {
+            const int part = c.next++;
+            copies.erase(std::find(copies.begin(), copies.end(), &c));
+            if (c.next < PARTS) copies.push_back(&c);   // behind the others
+            lk.unlock();
+            (*c.job)(part, PARTS);
+            lk.lock();
+            if (++c.done == PARTS) done.notify_all();
         }
-        wake_.notify_all();
-        for (auto& t : workers_) t.join();
-    }
-    void work(int part) {
-        uint64_t seen = 0;
-        for (;;) {
-            const std::function<void(int, int)>* job;
-            int parts;
-            {
-                std::unique_lock<std::mutex> lk(mu_);
-                wake_.wait(lk, [&] { return stop_ || round_ != seen; });
-                if (stop_) return;
-                seen = round_;
-                job = job_;
-                parts = parts_;
-            }
-            (*job)(part, parts);
-            {
-                std::lock_guard<std::mutex> lk(mu_);
-                if (--left_ == 0) done_.notify_one();
+        void work() {
+            std::unique_lock<std::mutex> lk(mu);
+            for (;;) {
+                wake.wait(lk, [&] { return stop || !copies.empty(); });
+                if (stop) return;
+                take(lk, *copies.front());
             }
         }
-    }
-    std::mutex use_, mu_;
-    std::condition_variable wake_, done_;
-    std::vector<std::thread> workers_;
-    const std::function<void(int, int)>* job_ = nullptr;
-    int parts_ = 0, left_ = 0;
-    uint64_t round_ = 0;
-    bool stop_ = false;
+    };
+    const pid_t pid_ = getpid();
+    std::unique_ptr<State> s_;
 };
 
 }  // namespace fdk

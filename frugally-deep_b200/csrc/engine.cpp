@@ -1,6 +1,5 @@
 // Executor: device contexts, weight upload, plan execution, predict_multi sharding.
 #include "engine.hpp"
-#include "copy_pool.hpp"
 #include "kernels.cuh"
 #include "plan_attrs.hpp"
 
@@ -102,6 +101,12 @@ Engine::~Engine() {
         if (c->fork_event) cudaEventDestroy(c->fork_event);
         if (c->join_event) cudaEventDestroy(c->join_event);
     }
+}
+
+CopyPool& Engine::copy_pool() {
+    std::lock_guard<std::mutex> lk(copy_pool_mu_);
+    if (!copy_pool_) copy_pool_ = CopyPool::shared();
+    return *copy_pool_;
 }
 
 void Engine::upload_weights(DeviceCtx& c) {
@@ -1521,7 +1526,7 @@ void Engine::run_block(DeviceCtx& c, const Plan& p, const std::vector<int64_t>& 
                             gather(b0, b1);
                             return;
                         }
-                        CopyPool::instance().run([&](int part, int parts) {
+                        copy_pool().run([&](int part, int parts) {
                             const size_t share = ((b1 - b0) / (size_t)parts + 4095) / 4096 * 4096;
                             const size_t p0 = std::min(b1, b0 + share * (size_t)part), p1 = part == parts - 1 ? b1 : std::min(b1, p0 + share);
                             if (p0 < p1) gather(p0, p1);

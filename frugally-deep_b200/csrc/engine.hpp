@@ -7,6 +7,7 @@
 #pragma once
 
 #include "common.hpp"
+#include "copy_pool.hpp"
 #include "growing_memory.hpp"
 #include "model.hpp"
 
@@ -247,10 +248,13 @@ private:
     void run_block(DeviceCtx& c, const Plan& p, const std::vector<int64_t>& sample_ids, const float* const* in_ptrs,
                    float* const* out_ptrs, const ByteScale* bytes = nullptr);
     void upload_weights(DeviceCtx& c);
+    CopyPool& copy_pool();
 
     LoadedModel lm_;
     EngineOptions opt_;
     std::vector<std::unique_ptr<DeviceCtx>> ctx_;
+    std::mutex copy_pool_mu_;
+    std::shared_ptr<CopyPool> copy_pool_;   // taken on first use, shared with the other models of the process
     std::mutex plan_mu_;
     std::map<std::string, std::shared_ptr<Plan>> plans_;
 };

@@ -275,3 +275,7 @@ def run_host_program(name, tmp_path, flags=()):
 
 def test_growing_memory(tmp_path):
     run_host_program("growing_memory", tmp_path)
+
+
+def test_copy_pool(tmp_path):
+    run_host_program("copy_pool", tmp_path, ["-pthread"])

@@ -6,7 +6,6 @@
 #include <algorithm>
 #include <atomic>
 #include <cmath>
-#include <cstdlib>
 #include <cstring>
 #include <thread>
 
@@ -1304,11 +1303,6 @@ void Engine::predict_batch_device(int dev_index, int64_t batch, const float* con
 // No address of the caller's is ever part of a recording.
 template <typename F>
 void Engine::replay(DeviceCtx& c, const Plan& p, int64_t batch, std::vector<const void*> where, bool host, float low, float high, cudaStream_t s, F&& queue) {
-    static const bool enabled = [] { const char* v = getenv("FDK_PREDICT_GRAPH"); return !(v && *v == '0'); }();
-    if (!enabled) {
-        queue(s);
-        return;
-    }
     where.push_back(c.arena);
     where.push_back(c.workspace);
     const uint64_t memory = c.memory_moves, staging = host ? c.staging_moves : 0;

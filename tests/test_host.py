@@ -279,3 +279,9 @@ def test_growing_memory(tmp_path):
 
 def test_copy_pool(tmp_path):
     run_host_program("copy_pool", tmp_path, ["-pthread"])
+
+
+def test_predict_calls_read_no_environment():
+    """How a call is launched depends on the call alone: no switch of the whole process."""
+    with open(os.path.join(ROOT, "frugally-deep_b200", "csrc", "engine.cpp")) as f:
+        assert "getenv" not in f.read()

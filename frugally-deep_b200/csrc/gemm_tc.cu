@@ -1672,7 +1672,13 @@ constexpr int LQ_THREADS = 256;
 constexpr int LQ_UNITS = TC_GROUP * TC_BK;    // units of h per CTA: one accumulator group
 constexpr int LQ_GROUPS = 8;                  // most groups: 512 units (more would not fit the SMs but for a few sizes)
 constexpr int LQ_W_BYTES = TC_GROUP * 2 * 128 * TC_BK * 4;
-constexpr int LQ_SMEM = LQ_W_BYTES + LQ_ROWS * LQ_UNITS * 4 + 64;
+constexpr int LQ_SMEM_USED = LQ_W_BYTES + LQ_ROWS * LQ_UNITS * 4 + 64;
+// More than half of an SM's shared memory, so that no two of these CTAs share an SM.  The device guarantees that all CTAs of
+// a cooperative launch are resident as far as shared memory and registers go, not tensor memory: where other streams leave
+// few SMs free, three CTAs on one SM would want 768 of its 512 columns, and the third could not start while the others
+// wait for it at the barrier.
+constexpr int LQ_SMEM = 116 * 1024;
+static_assert(LQ_SMEM_USED <= LQ_SMEM && 2 * LQ_SMEM > 228 * 1024, "one CTA per SM");
 constexpr int LQ_ITEMS = LQ_ROWS * LQ_UNITS / LQ_THREADS;   // cells per thread
 
 struct LstmSeqParams {

@@ -1296,3 +1296,29 @@ def test_recorded_calls_forget_memory_that_was_given_back(built_library):
             m.predict_batch_device([d_in.data_ptr()], [[32, 32, 3]], 10 ** 8, [d_out.data_ptr()])   # terabytes
         call(1)
         call(200)
+
+
+def test_lstm_in_one_launch_beside_other_work(built_library):
+    """Two models' LSTM layers, whose CTAs meet at a barrier of the whole launch, beside a third model that keeps the SMs busy, on
+    three streams: every call gives what it gives alone."""
+    import torch
+    lstm = model_text(mw.build_text_lstm(seq_len=20, vocab=50, dim=32, units=512))
+    ms = [fdeep_b200.read_model_from_string(lstm, verify=False) for _ in range(2)]
+    busy, _ = load(mw.build_resnet50(size=64, width=32, classes=10, top="linear"), True)
+    x = [np.random.default_rng(i).integers(1, 50, size=(4, 20)).astype(np.float32) for i in range(2)]
+    want = [m.predict_batch([v])[0] for m, v in zip(ms, x)]
+    img = torch.from_numpy(mw.inputs_resnet50(32, size=64)).cuda()
+    img_out = torch.empty((32, 10), device="cuda")
+    d_in = [torch.from_numpy(v).cuda() for v in x]
+    streams = [torch.cuda.Stream() for _ in range(3)]
+    for rep in range(10):
+        d_out = [torch.zeros(w.shape, device="cuda") for w in want]
+        torch.cuda.synchronize()
+        for k in range(4):
+            busy.predict_batch_device([img.data_ptr()], [[64, 64, 3]], 32, [img_out.data_ptr()], stream=streams[2].cuda_stream)
+            for i, m in enumerate(ms):
+                m.predict_batch_device([d_in[i].data_ptr()], [[20]], 4, [d_out[i].data_ptr()], stream=streams[i].cuda_stream)
+        torch.cuda.synchronize()
+        for i, m in enumerate(ms):
+            m.sync()
+            np.testing.assert_array_equal(d_out[i].cpu().numpy(), want[i], err_msg=f"round {rep}, model {i}")

@@ -904,14 +904,17 @@ struct Exec {
                     r = Rec{"gemm", L.name, "tc sequence", nullptr, nullptr, 2.0 * (double)(B * T) * gu * U, B * T, gu, U};
                     rec_begin(r);
                 }
-                launch_lstm_sequence(c.w.base + c.w.big_offset[(size_t)L.w_rec], c.w.base + c.w.small_offset[(size_t)L.w_rec], L.kdim, X, parts,
-                                     c.grid_barrier, L.flag_b ? tptr(o.out[1]) : nullptr, L.flag_b ? tptr(o.out[2]) : nullptr, out, L.flag_a != 0, L.reverse != 0, B, T, U, s);
-                if (prof) {
-                    FDK_CUDA(cudaEventRecord(r.b, s));
-                    prof->push_back(r);
+                if (launch_lstm_sequence(c.w.base + c.w.big_offset[(size_t)L.w_rec], c.w.base + c.w.small_offset[(size_t)L.w_rec], L.kdim, X, parts,
+                                         c.grid_barrier, L.flag_b ? tptr(o.out[1]) : nullptr, L.flag_b ? tptr(o.out[2]) : nullptr, out,
+                                         L.flag_a != 0, L.reverse != 0, B, T, U, s)) {
+                    if (prof) {
+                        FDK_CUDA(cudaEventRecord(r.b, s));
+                        prof->push_back(r);
+                    }
+                    c.launches++;
+                    return;
                 }
-                c.launches++;
-                return;
+                if (prof) { cudaEventDestroy(r.a); cudaEventDestroy(r.b); }
             }
         }
         FDK_CUDA(cudaMemsetAsync(h, 0, sizeof(float) * (size_t)(B * U), s));

@@ -1905,7 +1905,7 @@ int64_t lstm_sequence_floats(int64_t B, int64_t T, int U, int64_t ldw, const voi
     return groups <= LQ_GROUPS && tiles * groups <= tc_sm_count() ? 2 * groups * B * 4 * U : 0;
 }
 
-void launch_lstm_sequence(const float* Wbig, const float* Wsmall, int64_t ldw, const float* x, float* parts, unsigned int* arrived, float* h, float* c,
+bool launch_lstm_sequence(const float* Wbig, const float* Wsmall, int64_t ldw, const float* x, float* parts, unsigned int* arrived, float* h, float* c,
                           float* out, bool every_step, bool reverse, int64_t B, int64_t T, int U, cudaStream_t s) {
     static std::mutex mu;
     static bool attr_set[64] = {};
@@ -1934,7 +1934,13 @@ void launch_lstm_sequence(const float* Wbig, const float* Wsmall, int64_t ldw, c
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    FDK_CUDA(cudaLaunchKernelEx(&cfg, lstm_sequence_kernel, mb, ms, prm));
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, lstm_sequence_kernel, mb, ms, prm);
+    if (e == cudaErrorCooperativeLaunchTooLarge) {
+        cudaGetLastError();
+        return false;
+    }
+    FDK_CUDA(e);
+    return true;
 }
 
 const int* gemm_tc_status_address() {

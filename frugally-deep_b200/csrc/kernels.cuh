@@ -96,9 +96,10 @@ int launch_gemm_tc_group_sums(const float* A, int64_t lda, const float* Wbig, co
                               cudaStream_t s);
 // All time steps of an LSTM layer (tanh / sigmoid) on at most 8 sequences in one launch, results as step by step.  x: gate
 // inputs [B][T][4U], bias included; parts: lstm_sequence_floats floats (0: not this form); arrived: one word of the caller's;
-// h, c: [B][U] last states (both or neither); out: [B][T][U] with every_step, else [B][U].
+// h, c: [B][U] last states (both or neither); out: [B][T][U] with every_step, else [B][U].  False (nothing launched): the
+// stream may not use as many SMs as the launch needs at once (a partition of the device).
 int64_t lstm_sequence_floats(int64_t B, int64_t T, int U, int64_t ldw, const void* W);
-void launch_lstm_sequence(const float* Wbig, const float* Wsmall, int64_t ldw, const float* x, float* parts, unsigned int* arrived, float* h, float* c,
+bool launch_lstm_sequence(const float* Wbig, const float* Wsmall, int64_t ldw, const float* x, float* parts, unsigned int* arrived, float* h, float* c,
                           float* out, bool every_step, bool reverse, int64_t B, int64_t T, int U, cudaStream_t s);
 // One LSTM time step in one launch: z = h U + x (x = this step's rows of the input product, bias included) never
 // leaves the SM; the epilogue applies the cell (tanh / sigmoid) and writes c in place, the new h to h_next (a buffer

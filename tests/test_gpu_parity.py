@@ -1322,3 +1322,40 @@ def test_lstm_in_one_launch_beside_other_work(built_library):
         for i, m in enumerate(ms):
             m.sync()
             np.testing.assert_array_equal(d_out[i].cpu().numpy(), want[i], err_msg=f"round {rep}, model {i}")
+
+
+def test_lstm_on_a_partition_of_the_device(built_library):
+    """All steps of an LSTM in one launch need 128 SMs at once; on a stream that may use 32 of them the layer runs step by step."""
+    import torch
+    driver = pytest.importorskip("cuda.bindings.driver")
+
+    def ok(r):
+        assert r[0] == driver.CUresult.CUDA_SUCCESS, r
+        return r[1] if len(r) == 2 else r[1:]
+
+    torch.zeros(1, device="cuda")
+    text = model_text(mw.build_text_lstm(seq_len=12, vocab=50, dim=32, units=512))
+    m, alone = (fdeep_b200.read_model_from_string(text, verify=False) for _ in range(2))
+    x = np.random.default_rng(1).integers(1, 50, size=(3, 12)).astype(np.float32)
+    want = alone.predict_batch([x])[0]
+    dev = ok(driver.cuDeviceGet(0))
+    sms = ok(driver.cuDeviceGetDevResource(dev, driver.CUdevResourceType.CU_DEV_RESOURCE_TYPE_SM))
+    groups, n, rest = ok(driver.cuDevSmResourceSplitByCount(1, sms, 0, 32))
+    desc = ok(driver.cuDevResourceGenerateDesc([groups[0]], 1))
+    part = ok(driver.cuGreenCtxCreate(desc, dev, driver.CUgreenCtxCreate_flags.CU_GREEN_CTX_DEFAULT_STREAM))
+    stream = ok(driver.cuGreenCtxStreamCreate(part, driver.CUstream_flags.CU_STREAM_NON_BLOCKING, 0))
+    try:
+        d_in, d_out = torch.from_numpy(x).cuda(), torch.zeros(want.shape, device="cuda")
+        torch.cuda.synchronize()
+        for rep in range(3):
+            d_out.zero_()
+            torch.cuda.synchronize()
+            m.predict_batch_device([d_in.data_ptr()], [[12]], 3, [d_out.data_ptr()], stream=int(stream))
+            torch.cuda.synchronize()
+            m.sync()
+            np.testing.assert_array_equal(d_out.cpu().numpy(), want)
+    finally:
+        torch.cuda.synchronize()
+        del m
+        driver.cuStreamDestroy(stream)
+        driver.cuGreenCtxDestroy(part)

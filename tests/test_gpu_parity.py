@@ -1039,8 +1039,9 @@ def test_category_encoding_value_outside_raises(built_library):
 
 
 # (input side, channels, filters, kernel, stride): k blocks 10 (ragged last), 18 with a partial channel chunk, 72, 16, 50;
-# columns that are no multiple of 32 or 64; one row of the tile, one partial tile, several tiles
-SPLIT_SHAPES = [(1, 300, 68, 1, 1), (7, 40, 256, 3, 1), (7, 256, 512, 3, 1), (14, 512, 36, 1, 1), (15, 64, 100, 5, 2)]
+# columns that are no multiple of 32 or 64; one row of the tile, one partial tile, several tiles; one k block per filter row
+# (three input channels: the row-window form)
+SPLIT_SHAPES = [(1, 300, 68, 1, 1), (7, 40, 256, 3, 1), (7, 256, 512, 3, 1), (14, 512, 36, 1, 1), (15, 64, 100, 5, 2), (16, 3, 64, (12, 7), 1)]
 
 
 @pytest.mark.parametrize("side,cin,cout,k,stride", SPLIT_SHAPES)
@@ -1053,7 +1054,8 @@ def test_few_rows_spread_over_the_k_blocks(built_library, side, cin, cout, k, st
     rng = np.random.default_rng(side * 1000 + cin + cout)
     b = mw.ModelBuilder("m")
     i = b.input([side, side, cin])
-    kernel = rng.normal(size=(k, k, cin, cout)).astype(np.float32) / np.sqrt(k * k * cin)
+    kh, kw = k if isinstance(k, tuple) else (k, k)
+    kernel = rng.normal(size=(kh, kw, cin, cout)).astype(np.float32) / np.sqrt(kh * kw * cin)
     y = mw.conv2d(b, i, "c", kernel, rng.normal(size=cout).astype(np.float32), strides=stride, padding="same",
                   activation="sigmoid" if tail == "sigmoid" else "linear")
     out_side = -(-side // stride)
@@ -1073,7 +1075,7 @@ def test_few_rows_spread_over_the_k_blocks(built_library, side, cin, cout, k, st
     want = oracle_outputs(text, pool[:1])
     np.testing.assert_array_equal(few[0], large[0][0])
     np.testing.assert_array_equal(few[0], large[many - many % 4 - 4][0])
-    assert_close(few[0], want[0][0], f"{side}x{side}x{cin} -> {cout}, {k}x{k}/{stride}, {tail}")
+    assert_close(few[0], want[0][0], f"{side}x{side}x{cin} -> {cout}, {kh}x{kw}/{stride}, {tail}")
     twice = m.predict_multi(pool[:1])   # (the group sums of the call before are still in the workspace)
     np.testing.assert_array_equal(few[0], twice[0][0])
     import torch
@@ -1114,23 +1116,39 @@ def test_lstm_step_on_group_sums(built_library, units, samples):
             assert_close(few[s][0], want[s][0], f"{units} units, sample {s}")
 
 
-@pytest.mark.parametrize("n", [1, 37, 341, 342])
-def test_device_calls_on_ever_new_buffers(built_library, n):
-    """predict_batch_device replays small calls (up to 4 MB of inputs and outputs, 341 samples here) on memory of the engine:
-    every call with other buffers and other values gives what the host path gives, and what lies around the output stays."""
+@pytest.mark.parametrize("at", [0, 16, 40], ids=["aligned", "16 bytes on", "40 bytes on"])
+@pytest.mark.parametrize("n", [1, 37, 340, 341])
+def test_device_calls_on_ever_new_buffers(built_library, n, at):
+    """predict_batch_device replays small calls (up to 4 MB of inputs and outputs: 340 samples here) on memory of the engine:
+    every call with other buffers and other values gives what the host path gives, and what lies around the output stays.  The
+    first call runs directly, the second is recorded, the others repeat the recording; an output that is not on a 16-byte
+    boundary (40 bytes on) is always queued directly, as 341 samples are."""
     import torch
     m, _ = load(mw.build_small_cnn(), True)
-    for rep in range(4):
+    alone, _ = load(mw.build_small_cnn(), True)
+    kept = []   # every call has buffers of its own
+    for rep in range(5):
         x = np.random.default_rng(100 * n + rep).random((n, 32, 32, 3), dtype=np.float32)
-        d_in = torch.from_numpy(x).cuda()
-        d_out = torch.full((n + 2, 10), -7.0, device="cuda")
+        d_in, d_out = torch.from_numpy(x).cuda(), torch.full((10 * n + 32,), -7.0, device="cuda")
+        kept.append((d_in, d_out))
         torch.cuda.synchronize()
-        m.predict_batch_device([d_in.data_ptr()], [[32, 32, 3]], n, [d_out[1:].data_ptr() if rep % 2 else d_out.data_ptr()])
+        m.predict_batch_device([d_in.data_ptr()], [[32, 32, 3]], n, [d_out.data_ptr() + at])
         m.sync()
         got = d_out.cpu().numpy()
-        first = 1 if rep % 2 else 0   # (40 bytes on: not 16-byte aligned)
-        np.testing.assert_array_equal(got[first:first + n], m.predict_batch([x])[0])
-        assert (np.delete(got, np.s_[first:first + n], axis=0) == -7.0).all()
+        first = at // 4
+        np.testing.assert_array_equal(got[first:first + 10 * n].reshape(n, 10), alone.predict_batch([x])[0], err_msg=f"call {rep}")
+        assert (np.delete(got, np.s_[first:first + 10 * n]) == -7.0).all()
+
+
+def test_recorded_byte_calls_keep_their_range(built_library):
+    """Byte inputs on one plan and batch with two ranges in turn: the range belongs to what is recorded."""
+    m, _ = load(mw.build_small_cnn(), True)
+    x = [np.random.default_rng(rep).integers(0, 256, size=(6, 32, 32, 3), dtype=np.uint8) for rep in range(5)]
+    for rep in range(5):
+        for low, high in ((0.0, 1.0), (-1.0, 1.0)):
+            floats = x[rep].astype(np.float32) * np.float32((np.float32(high) - np.float32(low)) / np.float32(255)) + np.float32(low)
+            got = m.predict_batch([x[rep]], bytes_range=(low, high))[0]
+            np.testing.assert_allclose(got, m.predict_batch([floats])[0], rtol=1e-5, atol=1e-6, err_msg=f"call {rep}, range {low}")
 
 
 @pytest.mark.parametrize("side,channels", [((3, 3), 16), ((8, 16), 33), ((3, 43), 64), ((17, 23), 1280)])

@@ -1299,11 +1299,16 @@ void Engine::predict_batch_device(int dev_index, int64_t batch, const float* con
     if (live) mark_use(c, s);
 }
 
-// A call repeated with the same plan and batch (and the engine's buffers where they were) costs one graph launch instead of the launches of the plan (60 to
-// 800 of them, 3 to 6 us of host time each with their tensor maps, and gaps between short kernels).  The first call of a kind
-// runs directly (every buffer reaches its size), the second one is recorded.  At most 32 calls are kept per device; the
-// addresses of the staging buffers, the arena and the workspace belong to the key because other calls may make them move.
-// No address of the caller's is ever part of a recording.
+// A call repeated with the same plan and batch (and the engine's buffers where they were) costs one graph launch instead of
+// the launches of the plan (60 to 800 of them, 3 to 6 us of host time each with their tensor maps, and gaps between short
+// kernels).  The first calls of a kind run directly (every buffer reaches its size), the RECORD_AT-th one is recorded: that
+// costs as much as 4 to 16 calls gain by it (direct / recording / replayed: small CNN 87 / 170 / 70 us, MobileNetV2 on a few
+// images of side 96 457 / 789 / 386, 40 texts of 160 words 3183 / 7073 / 2900), so a kind that comes only a few times, such as
+// one of many text lengths, is better off without.  At most 32 kinds are kept per device; the addresses of the staging
+// buffers, the arena and the workspace belong to the key because other calls may make them move.  No address of the
+// caller's is ever part of a recording.
+static constexpr int RECORD_AT = 6;
+
 template <typename F>
 void Engine::replay(DeviceCtx& c, const Plan& p, int64_t batch, std::vector<const void*> where, bool host, float low, float high, cudaStream_t s, F&& queue) {
     where.push_back(c.arena);
@@ -1329,7 +1334,7 @@ void Engine::replay(DeviceCtx& c, const Plan& p, int64_t batch, std::vector<cons
         return;
     }
     r->last_use = ++c.call_clock;
-    if (!r->exec && !r->unusable) {
+    if (!r->exec && !r->unusable && ++r->calls >= RECORD_AT) {
         const int64_t before = c.launches;
         cudaGraph_t graph = nullptr;
         FDK_CUDA(cudaStreamBeginCapture(c.record_stream, cudaStreamCaptureModeRelaxed));

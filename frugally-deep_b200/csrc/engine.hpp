@@ -85,6 +85,7 @@ struct RecordedCall {
     float low = 0.f, high = 0.f;
     cudaGraphExec_t exec = nullptr;
     int64_t launches = 0;
+    int calls = 1;
     uint64_t last_use = 0;
     bool unusable = false;             // could not be recorded: launch directly
 };

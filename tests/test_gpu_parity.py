@@ -1121,13 +1121,13 @@ def test_lstm_step_on_group_sums(built_library, units, samples):
 def test_device_calls_on_ever_new_buffers(built_library, n, at):
     """predict_batch_device replays small calls (up to 4 MB of inputs and outputs: 340 samples here) on memory of the engine:
     every call with other buffers and other values gives what the host path gives, and what lies around the output stays.  The
-    first call runs directly, the second is recorded, the others repeat the recording; an output that is not on a 16-byte
+    first calls run directly, the sixth is recorded, the others repeat the recording; an output that is not on a 16-byte
     boundary (40 bytes on) is always queued directly, as 341 samples are."""
     import torch
     m, _ = load(mw.build_small_cnn(), True)
     alone, _ = load(mw.build_small_cnn(), True)
     kept = []   # every call has buffers of its own
-    for rep in range(5):
+    for rep in range(9):
         x = np.random.default_rng(100 * n + rep).random((n, 32, 32, 3), dtype=np.float32)
         d_in, d_out = torch.from_numpy(x).cuda(), torch.full((10 * n + 32,), -7.0, device="cuda")
         kept.append((d_in, d_out))
@@ -1143,8 +1143,8 @@ def test_device_calls_on_ever_new_buffers(built_library, n, at):
 def test_recorded_byte_calls_keep_their_range(built_library):
     """Byte inputs on one plan and batch with two ranges in turn: the range belongs to what is recorded."""
     m, _ = load(mw.build_small_cnn(), True)
-    x = [np.random.default_rng(rep).integers(0, 256, size=(6, 32, 32, 3), dtype=np.uint8) for rep in range(5)]
-    for rep in range(5):
+    x = [np.random.default_rng(rep).integers(0, 256, size=(6, 32, 32, 3), dtype=np.uint8) for rep in range(9)]
+    for rep in range(9):
         for low, high in ((0.0, 1.0), (-1.0, 1.0)):
             floats = x[rep].astype(np.float32) * np.float32((np.float32(high) - np.float32(low)) / np.float32(255)) + np.float32(low)
             got = m.predict_batch([x[rep]], bytes_range=(low, high))[0]
@@ -1194,7 +1194,7 @@ def test_clipped_relu_keeps_what_is_not_a_number(built_library, cin, cout, n, ta
 
 
 def test_sync_while_another_thread_records(built_library):
-    """Two threads make device calls of ever new sizes on one model, the second call of each being recorded, and wait with sync();
+    """Two threads make device calls of ever new sizes on one model, the sixth call of each being recorded, and wait with sync();
     a third waits all the time.  Nobody gets an error and every result is that of a call on its own."""
     import threading
     import torch
@@ -1211,7 +1211,7 @@ def test_sync_while_another_thread_records(built_library):
             d_out = torch.zeros((len(x), 10), device="cuda")
             torch.cuda.synchronize()
             for n in sizes[t::2]:
-                for rep in range(4):
+                for rep in range(8):
                     m.predict_batch_device([d_in[rep % 3:].data_ptr()], [[32, 32, 3]], n, [d_out.data_ptr()])
                     m.sync()
                     np.testing.assert_array_equal(d_out[:n].cpu().numpy(), want[rep % 3:rep % 3 + n], err_msg=f"{n} samples, call {rep}")
@@ -1259,7 +1259,7 @@ def test_outputs_that_share_memory_or_lie_on_the_host(built_library, n):
         return torch.zeros((n, 12, 12, 16), **where)
 
     want = call(new(device="cuda"), new(device="cuda"))
-    for rep in range(3):
+    for rep in range(8):
         shift = n // 2   # the later output starts in the middle of the earlier one, which is read after its first tiles are written
         both = torch.zeros((n + shift, 12, 12, 16), device="cuda")
         np.testing.assert_array_equal(call(both[:n], both[shift:])[1], want[1])
@@ -1308,7 +1308,7 @@ def test_recorded_calls_forget_memory_that_was_given_back(built_library):
         np.testing.assert_array_equal(d_out[:n].cpu().numpy(), want[:n])
 
     for rep in range(3):
-        for _ in range(3):
+        for _ in range(8):
             call(200)
         with pytest.raises(fdeep_b200.FdeepError, match="arena allocation"):
             m.predict_batch_device([d_in.data_ptr()], [[32, 32, 3]], 10 ** 8, [d_out.data_ptr()])   # terabytes
@@ -1365,7 +1365,7 @@ def test_lstm_on_a_partition_of_the_device(built_library):
     try:
         d_in, d_out = torch.from_numpy(x).cuda(), torch.zeros(want.shape, device="cuda")
         torch.cuda.synchronize()
-        for rep in range(3):
+        for rep in range(8):
             d_out.zero_()
             torch.cuda.synchronize()
             m.predict_batch_device([d_in.data_ptr()], [[12]], 3, [d_out.data_ptr()], stream=int(stream))
@@ -1377,3 +1377,22 @@ def test_lstm_on_a_partition_of_the_device(built_library):
         del m
         driver.cuStreamDestroy(stream)
         driver.cuGreenCtxDestroy(part)
+
+
+def test_a_kind_of_call_that_comes_twice_is_not_recorded(built_library):
+    """Recording a call takes longer than running it (two LSTM layers of 40 texts: 7.1 ms where a direct call takes 3.2), so the
+    second call of a kind is about as fast as the first."""
+    import time
+    import torch
+    m = fdeep_b200.read_model_from_string(model_text(mw.build_text_lstm(seq_len=None, vocab=50, dim=32, units=512)), verify=False)
+    m.predict_batch([np.ones((64, 200), np.float32)])
+    times = []
+    for steps in range(150, 158):
+        x, out = torch.ones((40, steps), device="cuda"), torch.empty((40, 1), device="cuda")
+        torch.cuda.synchronize()
+        for call in range(2):
+            t = time.perf_counter()
+            m.predict_batch_device([x.data_ptr()], [[steps]], 40, [out.data_ptr()])
+            m.sync()
+            times.append(time.perf_counter() - t)
+    assert np.median(times[1::2]) < 1.5 * np.median(times[::2]), times

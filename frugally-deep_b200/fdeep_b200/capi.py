@@ -257,8 +257,9 @@ class Model:
             return outs
         # one array of addresses per call, written without a Python loop over the samples
         row = np.arange(ns, dtype=np.uint64)[:, None]
-        in_ptrs = np.array([_address(a) for a in arrs], np.uint64) + row * np.array([a.strides[0] for a in arrs], np.uint64)
-        out_ptrs = np.array([_address(a) for a in outs], np.uint64) + row * np.array([a.strides[0] for a in outs], np.uint64)
+        # (a.strides[0] is no guide: the only sample of a contiguous array may have any stride, a negative one included)
+        in_ptrs = np.array([_address(a) for a in arrs], np.uint64) + row * np.array([a.nbytes // ns for a in arrs], np.uint64)
+        out_ptrs = np.array([_address(a) for a in outs], np.uint64) + row * np.array([a.nbytes // ns for a in outs], np.uint64)
         dims = np.tile(np.array(one, np.int64), ns)
         ranks = np.tile(np.array(one_rank, np.intc), ns)
         vpp = C.POINTER(C.c_void_p)

@@ -1396,3 +1396,13 @@ def test_a_kind_of_call_that_comes_twice_is_not_recorded(built_library):
             m.sync()
             times.append(time.perf_counter() - t)
     assert np.median(times[1::2]) < 1.5 * np.median(times[::2]), times
+
+
+def test_batch_of_one_with_a_stride_of_its_own(built_library):
+    """A batch array of one sample may come with any batch stride and still be contiguous: reversed, broadcast, every other row."""
+    m, _ = load(mw.build_small_cnn(), True)
+    x = mw.inputs_small_cnn(3)
+    want = m.predict_batch([x])[0]
+    for one in (x[:1][::-1], np.broadcast_to(x[0], (1, 32, 32, 3)), x[::2][:1], x[2::-2][1:]):
+        np.testing.assert_array_equal(m.predict_batch([one])[0], want[:1])
+    np.testing.assert_array_equal(m.predict_batch([x[::-1]])[0], want[::-1])

@@ -1255,13 +1255,14 @@ void Engine::predict_batch_device(int dev_index, int64_t batch, const float* con
     };
     // A small call is replayed on memory of the engine, one copy in and one out per tensor: what is recorded knows nothing of
     // the caller's buffers, so new ones cost no more than the last call's.  Above DEVICE_STAGE_FLOATS (4 MB: a copy of about
-    // 3 us, 60 launches cost 200 us of host time) the device is busy for longer than the launches take to queue.
+    // 3 us, 60 launches cost 200 us of host time) the device is busy for longer than the launches take to queue.  An input that
+    // is not given (nothing that is asked for reads it) cannot be copied: direct.
     bool staged = live && !profile && !kv;
     int64_t floats = 0;
     auto reserve = [&](const void* q, int64_t n) {
         const int64_t at = floats;
         floats += round_up64(n, 64);
-        staged = staged && (reinterpret_cast<uintptr_t>(q) & 15) == 0 && floats <= DEVICE_STAGE_FLOATS;   // odd addresses: as they always were
+        staged = staged && q && (reinterpret_cast<uintptr_t>(q) & 15) == 0 && floats <= DEVICE_STAGE_FLOATS;   // odd addresses: as they always were
         return at;
     };
     std::vector<int64_t> in_at, out_at;

@@ -1406,3 +1406,19 @@ def test_batch_of_one_with_a_stride_of_its_own(built_library):
     for one in (x[:1][::-1], np.broadcast_to(x[0], (1, 32, 32, 3)), x[::2][:1], x[2::-2][1:]):
         np.testing.assert_array_equal(m.predict_batch([one])[0], want[:1])
     np.testing.assert_array_equal(m.predict_batch([x[::-1]])[0], want[::-1])
+
+
+def test_device_call_without_an_input_that_nothing_reads(built_library):
+    """An input that is handed through to an output nobody wants may be missing."""
+    import torch
+    rng = np.random.default_rng(2)
+    b = mw.ModelBuilder("m")
+    i, j = b.input([8]), b.input([5])
+    y = mw.dense(b, i, "d", rng.normal(size=(8, 4)).astype(np.float32), None)
+    m = fdeep_b200.read_model_from_string(model_text(b.to_json([y, j], [[4], [5]])), verify=False)
+    x, out = torch.randn((3, 8), device="cuda"), torch.zeros((3, 4), device="cuda")
+    torch.cuda.synchronize()
+    want = m.predict_multi([[v, np.zeros(5, np.float32)] for v in x.cpu().numpy()])
+    m.predict_batch_device([x.data_ptr(), 0], [[8], [5]], 3, [out.data_ptr(), 0])
+    m.sync()
+    np.testing.assert_array_equal(out.cpu().numpy(), np.stack([w[0] for w in want]))

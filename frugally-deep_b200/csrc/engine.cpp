@@ -1364,7 +1364,10 @@ void Engine::replay(DeviceCtx& c, const Plan& p, int64_t batch, std::vector<cons
     c.launches += r->launches;
 }
 
-// Inputs up to this size are fetched from page-locked memory by a kernel (below).
+// Inputs up to this size are fetched from page-locked memory by a kernel (below).  Small CNN from pageable memory, fetched /
+// copied: 12 KB 79 / 87 us, 360 KB 133 / 150, 600 KB 145 / 157, 960 KB 182 / 199; the forms cross later (1440 KB 266 / 430,
+// 2880 KB 494 / 540, 5760 KB 1010 / 910).  A page-locked input could be copied without being gathered first, which is the
+// better form from 100 KB on (100 KB 102 / 103, 360 KB 132 / 110, 960 KB 181 / 160).
 static constexpr int64_t FETCH_LIMIT = 1 << 20;
 
 // Whether memory of the caller is page-locked, so that a copy from it is one DMA.
@@ -1498,7 +1501,7 @@ void Engine::run_block(DeviceCtx& c, const Plan& p, const std::vector<int64_t>& 
                 if (cnb == 0) continue;
                 cudaStream_t cs = n_chunks > 1 ? c.copy_stream : c.stream;
                 // A small block goes through page-locked memory that the first kernel reads itself: many loads in flight across
-                // the bus from the start, where a copy engine took 103 us for the 602 KB of one 224 x 224 image.
+                // the bus from the start, without the hop to a copy engine.
                 const bool tiny = n_chunks == 1 && in_bytes <= FETCH_LIMIT;
                 std::vector<const float*> d_in(n_in);
                 std::vector<int64_t> at(n_in);   // offset of every input in the staging buffers

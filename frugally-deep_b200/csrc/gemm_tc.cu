@@ -256,7 +256,7 @@ struct TcParams {
     int tma_epi;                      // 1: output (and residual) rows are 16-byte aligned: TMA epilogue
     int runs, kb_run;                 // PARTS: runs per tile, k blocks per run (a multiple of TC_GROUP)
     EpiDev epi;
-    // LSTM step (kernel instance with CELL = true): state tensors [B][cell_U]; cell_out may be null
+    // LSTM step (kernel instance TC_CELL): state tensors [B][cell_U]; cell_out may be null
     float* cell_c;
     float* cell_h;
     float* cell_out;
@@ -1414,7 +1414,7 @@ void launch_conv_tc(const float* in, const ConvTcGeom& g, const float* Wbig, con
                     int N, const Epilogue& epilogue, cudaStream_t s) {
     // With nothing between the two activations (no BatchNormalization, no residual) the first one may as well be the last: the
     // epilogue through shared memory and TMA knows only that one, and a ReLU in the first place took the path for odd rows
-    // (1048576 x 32 x 27: 0.59 ms there).
+    // (1048576 x 32 x 27: 0.59 ms there, 0.17 here).  A ReLU in front of a BatchNormalization still takes that path.
     Epilogue e = epilogue;
     if (e.scale == nullptr && e.residual == nullptr && e.act2.none()) std::swap(e.act1, e.act2);
     // 64 columns per tile also when 128-column tiles would leave more than half of the SMs without one (few rows: a
@@ -1661,10 +1661,11 @@ void launch_lstm_step_tc(const float* h, const float* Wbig, const float* Wsmall,
 //   then finishes the cell of its own 64 units for every sequence from the sums of all groups, added in group order.
 // The tiles of a group do that last part redundantly, each with its own copy of c, which is what saves the second barrier
 // and the trip of h through memory; the sums alternate between two buffers, so that nobody overwrites what a slower CTA
-// still reads.  Same bits as the other forms.  Two layers of 512 units, 3 sequences of 120 steps: 2134 -> 1284 us, 5.1 us a
-// step; 8 sequences 1572 us, where 9, as two launches a step, take 1910.  At most 8: the sums that every CTA reads grow with
-// them (a step of 8 moves 8 MB through L2).
-// The CTAs wait for one another: cooperative launch.  Every wait is bounded (TC_WAIT_LIMIT_NS, status word).
+// still reads.  Same bits as the other forms.  Two layers of 512 units, 120 steps, this form / two launches a step: 1254 / 1862
+// us for 1 sequence, 1296 / 1808 for 3 (5.1 us a step), 1567 / 1914 for 8.  At most 8: the sums that every CTA reads grow
+// with them (a step of 8 moves 8 MB through L2), and built for 16 (four cells a thread instead of two) it takes 1476 for 3,
+// 1997 / 1892 for 9, 2039 / 2052 for 12 and 2371 / 2057 for 16.
+// The CTAs wait for one another: cooperative launch, one CTA per SM (LQ_SMEM).  Every wait is bounded (TC_WAIT_LIMIT_NS, status word).
 namespace {
 
 constexpr int LQ_ROWS = 8;                    // most sequences: the redundant part grows with them

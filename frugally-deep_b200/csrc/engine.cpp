@@ -62,7 +62,7 @@ Engine::Engine(LoadedModel&& lm, const std::vector<int>& devices, const EngineOp
         FDK_CUDA(cudaEventCreateWithFlags(&c->join_event, cudaEventDisableTiming));
         FDK_CUDA(cudaEventCreateWithFlags(&c->busy, cudaEventDisableTiming));
         FDK_CUDA(cudaMalloc(&c->d_err, 2 * sizeof(int)));
-        FDK_CUDA(cudaMemset(c->d_err, 0, 2 * sizeof(int)));
+        FDK_CUDA(cudaMemsetAsync(c->d_err, 0, 2 * sizeof(int), c->stream));   // waited for in upload_weights
         FDK_CUDA(cudaMalloc(&c->grid_barrier, sizeof(unsigned int)));
         FDK_CUDA(cudaMallocHost(&c->h_err, 8 * sizeof(int)));
         std::memset(c->h_err, 0, 8 * sizeof(int));
@@ -1605,7 +1605,7 @@ void Engine::run_block(DeviceCtx& c, const Plan& p, const std::vector<int64_t>& 
         } catch (...) {
             cudaStreamSynchronize(c.copy_stream);
             cudaStreamSynchronize(c.stream);
-            cudaMemset(c.d_err + 1, 0, sizeof(int));   // (the kernel that clears it may not have been launched)
+            cudaMemsetAsync(c.d_err + 1, 0, sizeof(int), c.stream);   // (the kernel that clears it may not have been launched)
             for (cudaEvent_t e : landed) if (e) cudaEventDestroy(e);
             throw;
         }

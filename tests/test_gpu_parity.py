@@ -1269,7 +1269,8 @@ def test_outputs_that_share_memory_or_lie_on_the_host(built_library, n):
         np.testing.assert_array_equal(got[1], want[1])
 
 
-def test_a_callers_graph_outlives_other_batches(built_library):
+@pytest.mark.parametrize("mode", ["relaxed", "global"])
+def test_a_callers_graph_outlives_other_batches(built_library, mode):
     """A device call on a few samples, captured by the caller, still gives its results after calls of other sizes, each of which
     needs more memory for the group sums of its products (and less of the other buffers than the first, large call)."""
     import torch
@@ -1280,7 +1281,7 @@ def test_a_callers_graph_outlives_other_batches(built_library):
     m.predict_batch([x[:1]])
     d_in, d_out = torch.from_numpy(x[:1]).cuda(), torch.zeros((1, 10), device="cuda")
     graph = torch.cuda.CUDAGraph()
-    with torch.cuda.graph(graph, capture_error_mode="relaxed"):
+    with torch.cuda.graph(graph, capture_error_mode=mode):
         m.predict_batch_device([d_in.data_ptr()], [[64, 64, 3]], 1, [d_out.data_ptr()], stream=torch.cuda.current_stream().cuda_stream)
     for n in (3, 7, 20):
         m.predict_batch([x[:n]])
@@ -1422,3 +1423,20 @@ def test_device_call_without_an_input_that_nothing_reads(built_library):
     m.predict_batch_device([x.data_ptr(), 0], [[8], [5]], 3, [out.data_ptr(), 0])
     m.sync()
     np.testing.assert_array_equal(out.cpu().numpy(), np.stack([w[0] for w in want]))
+
+
+def test_a_callers_graph_of_an_lstm(built_library):
+    """The LSTM in one launch (cooperative) inside a graph that a caller captured, replayed with other texts."""
+    import torch
+    m = fdeep_b200.read_model_from_string(model_text(mw.build_text_lstm(seq_len=20, vocab=50, dim=32, units=512)), verify=False)
+    x = np.random.default_rng(4).integers(1, 50, size=(4, 3, 20)).astype(np.float32)
+    want = [m.predict_batch([v])[0] for v in x]
+    d_in, d_out = torch.from_numpy(x[0]).cuda(), torch.zeros(want[0].shape, device="cuda")
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        m.predict_batch_device([d_in.data_ptr()], [[20]], 3, [d_out.data_ptr()], stream=torch.cuda.current_stream().cuda_stream)
+    for v, w in zip(x, want):
+        d_in.copy_(torch.from_numpy(v))
+        graph.replay()
+        torch.cuda.synchronize()
+        np.testing.assert_array_equal(d_out.cpu().numpy(), w)
